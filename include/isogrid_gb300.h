@@ -89,8 +89,9 @@ int igd_hpsi_agrid_host(int dtype, int closure, int nx, int ny, int nz, const vo
 
 /* Kernel selection for igd_hpsi_agrid (a test hook, per host thread): 0 = the
  * fastest applicable kernel (whole-row z-vectorised, then the tiled TMA
- * kernel, then the cp.async kernel), 1 = skip the whole-row kernel, 2 = the
- * cp.async kernel only.  No reference counterpart. */
+ * kernel, then the linear-tile kernel, then the cp.async kernel), 1 = skip the
+ * whole-row kernel, 2 = the cp.async kernel only, 3 = the linear-tile kernel
+ * first.  No reference counterpart. */
 int igd_hpsi_select(int path);
 /* Autotuner of the whole-row H.Psi kernel (process-wide; no reference
  * counterpart): mode 1 (default) times every orbitals-per-CTA choice (4, 2, 1)

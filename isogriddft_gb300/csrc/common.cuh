@@ -109,6 +109,12 @@ bool hpsi_agrid_krylov_applies(int nz, const void* coeffs);
 int hpsi_agrid_krylov(int nx, int ny, int nz, const float* coeffs, const float* psi, float* out, double kscale,
                       const float* dot_y, double* dot_acc, const int* skip, cudaStream_t st);
 
+// Linear-tile kernel of igd_hpsi_agrid (hpsi_agrid_lin.cu): FP64, and FP32 rows of any length
+// and alignment; -1 = not applicable (rows too long for a tile).
+int hpsi_agrid_lin_launch(int dtype, int closure, int nx, int ny, int nz, const void* coeffs, const void* veff,
+                          const void* psi, void* out, int nb, long long ostride, double kscale, double vscale,
+                          cudaStream_t st);
+
 // Whole-row z-vectorised fast path of igd_hpsi_agrid (hpsi_agrid_zvec.cu); -1 = not applicable.
 int hpsi_agrid_zvec_launch(int dtype, int closure, int nx, int ny, int nz, const void* coeffs, const void* veff,
                            const void* psi, void* out, int nb, long long ostride, double kscale, double vscale,

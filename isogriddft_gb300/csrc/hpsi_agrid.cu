@@ -348,7 +348,7 @@ using namespace igd;
 
 // Kernel selection (a test hook) of the calling host thread: 0 = fastest
 // applicable kernel, 1 = skip the whole-row kernel, 2 = the cp.async kernel
-// only.  IGD_HPSI_FALLBACK=1 in the environment starts every thread at 2.
+// only, 3 = the linear-tile kernel first.  IGD_HPSI_FALLBACK=1 in the environment starts every thread at 2.
 static thread_local int g_hpsi_path = -1;
 
 static int hpsi_path() {
@@ -360,7 +360,7 @@ static int hpsi_path() {
 }
 
 extern "C" int igd_hpsi_select(int path) {
-  if (path < 0 || path > 2) return IGD_ERR_ARG;
+  if (path < 0 || path > 3) return IGD_ERR_ARG;
   g_hpsi_path = path;
   return IGD_OK;
 }
@@ -395,6 +395,11 @@ extern "C" int igd_hpsi_agrid(int dtype, int closure, int nx, int ny, int nz, co
   const bool prod = closure == IGD_CLOSURE_PRODUCTION;
   cudaStream_t st = as_stream(stream);
   const int path = hpsi_path();
+  if (path == 3) {
+    const int t = hpsi_agrid_lin_launch(dtype, closure, nx, ny, nz, coeffs, veff, psi, out, nb, orbital_stride, kscale,
+                                        vscale, st);
+    if (t >= 0) return t;
+  }
   if (path == 0) {
     const int t = hpsi_agrid_zvec_launch(dtype, closure, nx, ny, nz, coeffs, veff, psi, out, nb, orbital_stride,
                                          kscale, vscale, st);
@@ -402,6 +407,14 @@ extern "C" int igd_hpsi_agrid(int dtype, int closure, int nx, int ny, int nz, co
   }
   if (path <= 1) {
     const int t = hpsi_agrid_tma_launch(dtype, closure, nx, ny, nz, coeffs, veff, psi, out, nb, orbital_stride, kscale,
+                                        vscale, st);
+    if (t >= 0) return t;
+  }
+  // FP64, and FP32 rows that the TMA kernels cannot take (their length or the data's alignment
+  // is not a multiple of 16 bytes).  What is left for the cp.async kernel: rows of more than 256
+  // points, FP64 scalings that are no power of two or with vscale != 1.
+  if (path != 2) {
+    const int t = hpsi_agrid_lin_launch(dtype, closure, nx, ny, nz, coeffs, veff, psi, out, nb, orbital_stride, kscale,
                                         vscale, st);
     if (t >= 0) return t;
   }
