@@ -105,10 +105,11 @@ int igd_hpsi_autotune(int mode);
  * returns the length written, or the full length when buf is null. */
 int igd_hpsi_autotune_report(char* buf, int len);
 /* Test hook: Gram kernel for the calling host thread (0 automatic, 1 tensor
- * pipe where it applies, 2 pipelined CUDA-core, 3 register-tiled CUDA-core).
- * No reference counterpart. */
+ * pipe where it applies (FP32), 2 pipelined CUDA-core, 3 register-tiled
+ * CUDA-core, 4 exact splitting on the tensor pipe (FP64)).  No reference
+ * counterpart. */
 int igd_gram_select(int path);
-/* Kernel that ran the calling thread's last igd_block_gram (1, 2, 3 as above). */
+/* Kernel that ran the calling thread's last igd_block_gram (1 to 4 as above). */
 int igd_gram_last_path(void);
 
 /* Legacy separable sinh grid, 7-point flux form with zero ghosts

@@ -8,6 +8,7 @@
 // FP32 data: products and per-thread sums (at most 64 points) in FP32, block
 // and cross-block accumulation in FP64; FP64 data: FP64 throughout.  Cross-block
 // sums are deterministic (per-block partials reduced in a second kernel).
+#include "blas64_split.cuh"
 #include "common.cuh"
 #include "gram_tc.cuh"
 #include "tma.cuh"
@@ -19,6 +20,17 @@ constexpr int GTH = 256;   // threads per Gram block
 constexpr long long kGramTcMinPoints = 1LL << 18;  // below this the CUDA-core kernels have less set-up
 thread_local int g_gram_path = 0;                   // igd_gram_select
 thread_local int g_gram_last = 0;                   // kernel of this thread's last Gram (1 tensor, 2 pipe, 3 tiled)
+// FP64: the splitting kernel takes about 22 clocks a point for every 16 x 24 outputs (splitting) plus
+// 8 (row exponents), the plain kernels 0.57 a point and output (FP64 pipe).  363609 points, plain /
+// split: 4 x 4 99 / 46 us (launch-bound plain grid), 8 x 8 99 / 48, 12 x 12 187 / 64, 21 x 21
+// 538 / 140, 34 x 34 1141 / 346; 2000003 points: 4 x 4 122 / 173, 8 x 8 376 / 202.  It would pay from
+// about a thousand points on (20001 points, 21 x 21: 72 / 29 us), but its correctly rounded sums
+// differ from the plain ones in the last bit, and on small grids an eigensolve of a closure that is
+// not self-adjoint turns that into 1e-8 of an unconverged orbital; below the size where the FP32
+// Gram changes kernels too, the plain sums and with them the recorded iterates are kept.
+inline bool gram64_split_pays(long long n, int a, int b) {
+  return n >= kGramTcMinPoints && 0.57 * a * b > 22.0 * ((a + 15) / 16) * ((b + 23) / 24) + 8.0;
+}
 constexpr int GPT = 64;    // points per thread and block column (FP32 partial sums stay short)
 
 // Register-tiled tall-skinny Gram.  Block (x, y): tile y of TR x TR outputs
@@ -255,7 +267,7 @@ __global__ void gram_reduce_kernel(int nblocks, int ab, const double* __restrict
 constexpr int RTH = 256;
 
 // out[j][p] (+)= sum_i A[i][p] C1[i][j] + sum_i B[i][p] C2[i][j] for j in
-// [j0, j0 + RC); RC in {4, 8, 16, 32} is the smallest that covers c (or 32).
+// [j0, j0 + RC), RC from rotate_dispatch.
 template <typename T, int RC>
 __global__ void __launch_bounds__(RTH) rotate_kernel(long long n, int a, const T* __restrict__ A, long long sa,
                                                      const double* __restrict__ C1, int b, const T* __restrict__ B,
@@ -323,10 +335,27 @@ int rotate_launch(long long n, int a, const T* A, long long sa, const double* C1
 template <typename T>
 int rotate_dispatch(long long n, int a, const T* A, long long sa, const double* C1, int b, const T* B, long long sb,
                     const double* C2, int c, T* out, long long so, int accumulate, cudaStream_t st) {
-  if (c <= 4) return rotate_launch<T, 4>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
-  if (c <= 8) return rotate_launch<T, 8>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
-  if (c <= 16) return rotate_launch<T, 16>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
-  return rotate_launch<T, 32>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
+  if constexpr (sizeof(T) == 8) {
+    // The FP64 pipe (two lanes per clock and SM) bounds this form, so no column is padded: equal
+    // tiles of at most 20 columns (40 accumulator registers), the width compiled in.  21 -> 20
+    // columns over 363609 points: one 32-column tile 424 us, 20 columns 269 us; 21 -> 1 with 4 columns 58
+    // us, with one 19 us.
+    const int tiles = (c + 19) / 20;
+    switch ((c + tiles - 1) / tiles) {
+#define IGD_ROT(RC) \
+  case RC: return rotate_launch<T, RC>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
+      IGD_ROT(1) IGD_ROT(2) IGD_ROT(3) IGD_ROT(4) IGD_ROT(5) IGD_ROT(6) IGD_ROT(7) IGD_ROT(8) IGD_ROT(9) IGD_ROT(10)
+      IGD_ROT(11) IGD_ROT(12) IGD_ROT(13) IGD_ROT(14) IGD_ROT(15) IGD_ROT(16) IGD_ROT(17) IGD_ROT(18) IGD_ROT(19)
+      IGD_ROT(20)
+#undef IGD_ROT
+    }
+    return IGD_ERR_ARG;
+  } else {
+    if (c <= 4) return rotate_launch<T, 4>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
+    if (c <= 8) return rotate_launch<T, 8>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
+    if (c <= 16) return rotate_launch<T, 16>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
+    return rotate_launch<T, 32>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
+  }
 }
 
 // Blocks (and per-block partials) of a Gram: one column slice of GTH x GPT
@@ -420,9 +449,9 @@ extern "C" int igd_precond_jacobi(int dtype, long long n, int k, const void* r, 
 
 // Gram kernel choice for the calling host thread (tests): 0 automatic, 1 the
 // tcgen05 kernel where it applies, 2 the pipelined CUDA-core kernel, 3 the
-// register-tiled kernel.
+// register-tiled kernel, 4 the FP64 splitting kernel (FP64 data).
 extern "C" int igd_gram_select(int path) {
-  if (path < 0 || path > 3) return IGD_ERR_ARG;
+  if (path < 0 || path > 4) return IGD_ERR_ARG;
   g_gram_path = path;
   return IGD_OK;
 }
@@ -432,7 +461,8 @@ extern "C" int igd_gram_last_path(void) { return g_gram_last; }
 
 extern "C" long long igd_block_gram_workspace_bytes(long long n, int a, int b) {
   if (n <= 0 || a <= 0 || b <= 0) return -1;
-  return (long long)gram_blocks(n) * a * b * (long long)sizeof(double);
+  // per-block partials (pairs in the FP64 splitting kernel), and that kernel's row exponents
+  return (2LL * gram_blocks(n) * a * b + (a + b + 1) / 2) * (long long)sizeof(double);
 }
 
 // out (a x b, FP64, row-major) [+]= A W B^T for row-major blocks A (a x n, row
@@ -458,6 +488,15 @@ extern "C" int igd_block_gram(int dtype, long long n, int a, const void* A, long
       return launch_status();
     }
     if (r != -1) return r;
+  }
+  if (dtype == IGD_F64 && (path == 4 || (path == 0 && gram64_split_pays(n, a, b)))) {
+    const int r = gram64_split_launch(n, a, static_cast<const double*>(A), sa, b, static_cast<const double*>(B), sb, w,
+                                      out, accumulate, reinterpret_cast<longlong2*>(part), gram_blocks(n),
+                                      reinterpret_cast<int*>(part + 2LL * gram_blocks(n) * a * b), st);
+    if (r != -1) {
+      g_gram_last = 4;
+      return r;
+    }
   }
   // the pipelined kernel when rows are 16-byte aligned and outputs <= 64 x 64, else the register-tiled one
   const int e = path == 3 ? -1

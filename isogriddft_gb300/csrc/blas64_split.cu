@@ -1,0 +1,330 @@
+// FP64 Gram products (K6) by exact splitting on the tensor cores.
+//
+// Reference: weighted_overlap_matrix (ks/eigensolver.py:246-272).
+//
+// GB300's FP64 pipe runs two lanes per clock and SM, so an FP64 Gram of 21 x 21 outputs costs 220
+// clocks of it per point.  Here every FP64 value becomes a fixed-point number of 63 bits relative to
+// the largest exponent of its row, and that seven balanced digits of nine bits, digits in
+// [-256, 255], which FP16 holds exactly (Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 95
+// (2012): error-free splitting into slices whose products accumulate without rounding).  The
+// products of two digits are integers of at most 2^16; an FP32 accumulator takes 256 of them
+// without rounding, so the sums of all digit pairs of one weight (28 pairs in seven levels; lower
+// ones are below 2^-58 of the largest product) are exact integers over a window of 32 points,
+// collected as int32 and turned into FP64 once per warp.  What is lost are bits below 2^-61 of the
+// row's largest value, where an FP64 sum rounds every product and partial sum to 2^-53: errors
+// against extended-precision sums are those of the plain kernels or smaller.  Splitting is integer
+// work on the otherwise idle ALUs (about 35 instructions a value) and bounds the kernel; the
+// products go through mma.sync m16n8k16 (FP16 in, FP32 out), whose fragments are the splitting's own
+// registers (the tensor pipe is a tenth busy: operands staged for tcgen05 would only add traffic).
+//
+// Measured, 363609 points, plain kernel / this one: 21 x 21 538 / 140 us, 34 x 34 1141 / 346 us; errors
+// against extended precision a quarter to all of the plain kernel's (tests/test_gram_fp64_split_gpu.py).
+#include <algorithm>
+
+#include <cuda_fp16.h>
+
+#include "blas64_split.cuh"
+
+namespace igd {
+namespace {
+
+constexpr int SL = 7;                                    // digits (slices) per value, levels of their products
+constexpr long long BIAS = 256LL * (((1LL << 62) - 1 + (1LL << 62)) / 511);  // sum of 256 * 512^k, k < 7
+static_assert(BIAS == 256LL * (1 + 512LL + 512LL * 512 + 512LL * 512 * 512 + 512LL * 512 * 512 * 512 +
+                               512LL * 512 * 512 * 512 * 512 + 512LL * 512 * 512 * 512 * 512 * 512),
+              "one balanced offset per digit");
+
+__device__ __forceinline__ int biased_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// x * 2^(61 - (emax - 1022)) truncated to an integer, plus the digit offsets; |x| < 2^(emax - 1022),
+// emax >= 1.
+__device__ __forceinline__ unsigned long long fixed63(double x, int emax) {
+  const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+  const unsigned long long mant = ((unsigned long long)((hi & 0xfffff) | (e ? 0x100000 : 0)) << 32) | (unsigned)__double2loint(x);
+  const int d = min(emax - max(e, 1), 63);  // subnormals have the exponent of the smallest normal
+  const long long m = (long long)((mant << 8) >> d), s = (long long)(hi >> 31);
+  return (unsigned long long)(((m ^ s) - s) + BIAS);
+}
+
+// Digits of two values, most significant first, as packed FP16 pairs (x0 in the low half).
+__device__ __forceinline__ void digits2(unsigned long long t0, unsigned long long t1, uint32_t (&d)[SL]) {
+  const unsigned l0 = (unsigned)t0, h0 = (unsigned)(t0 >> 32), l1 = (unsigned)t1, h1 = (unsigned)(t1 >> 32);
+  const __half2 off = __half2half2(__float2half(-1280.f));
+  auto pack = [&](unsigned a, unsigned b16) {  // 1024 + digit + 256, then exact subtraction
+    const unsigned v = (a & 0x1ffu) | (b16 & 0x1ff0000u) | 0x64006400u;
+    const __half2 r = __hadd2(*reinterpret_cast<const __half2*>(&v), off);
+    return *reinterpret_cast<const uint32_t*>(&r);
+  };
+  d[6] = pack(l0, l1 << 16);
+  d[5] = pack(l0 >> 9, l1 << 7);
+  d[4] = pack(l0 >> 18, l1 >> 2);
+  d[3] = pack(__funnelshift_r(l0, h0, 27), __funnelshift_r(l1, h1, 11));
+  d[2] = pack(h0 >> 4, h1 << 12);
+  d[1] = pack(h0 >> 13, h1 << 3);
+  d[0] = pack(h0 >> 22, h1 >> 6);
+}
+
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, "
+      "%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Seven level sums (weights 512^-l) as two integers of units 512^-2 and 512^-5, the last level
+// rounded to nearest (its floor, once per warp, showed as a bias of 2^-55 in the sum).
+__device__ __forceinline__ longlong2 halves(const int (&s)[SL]) {
+  return make_longlong2(((long long)s[0] << 18) + ((long long)s[1] << 9) + (long long)s[2],
+                        ((long long)s[3] << 18) + ((long long)s[4] << 9) + (long long)s[5] + ((s[6] + 256) >> 9));
+}
+// (hi 2^27 + lo) 2^shift, rounded once.
+__device__ __forceinline__ double join(long long hi, long long lo, int shift) {
+  const double h = (double)hi;
+  const long long rest = hi - (long long)h;  // what the conversion rounded off
+  return scalbn(fma(h, 134217728.0, fma((double)rest, 134217728.0, (double)lo)), shift);
+}
+
+// ------------------------------------------------------------------------------------- Gram
+// Largest biased exponent of every row of A and of w B (bounded by the factors' exponents);
+// rows of A first.  2047 marks a row with an infinity or a NaN.  A thread keeps the exponents of w
+// at its eight points while it runs over the rows (U loads in flight, five instructions a value).
+constexpr int EU = 8, ETH = 128, ER = 6;  // points per thread, threads, rows per CTA
+__global__ void __launch_bounds__(ETH) row_exponent_kernel(long long n, int a, const double* __restrict__ A,
+                                                           long long sa, int b, const double* __restrict__ B,
+                                                           long long sb, const double* __restrict__ w,
+                                                           int* __restrict__ emax) {
+  __shared__ int top[ER];
+  const int first = blockIdx.y * ER, past = min(a + b, first + ER);
+  if (threadIdx.x < ER) top[threadIdx.x] = 0;
+  __syncthreads();
+  const long long p0 = (long long)blockIdx.x * (ETH * EU) + threadIdx.x;
+  const bool whole = (long long)(blockIdx.x + 1) * (ETH * EU) <= n;
+  int off[EU], ew[EU];
+#pragma unroll
+  for (int u = 0; u < EU; ++u) {
+    off[u] = whole || p0 + ETH * u < n ? ETH * u : 0;  // threads past the end repeat a point
+    const long long p = min(p0 + off[u], n - 1);
+    off[u] = (int)(p - p0);
+    ew[u] = w ? max(biased_exponent(__ldg(w + p)), 1) - 1022 : 1;
+  }
+  const bool wbad = [&] {
+    bool f = false;
+#pragma unroll
+    for (int u = 0; u < EU; ++u) f |= ew[u] == 0x7ff - 1022;
+    return f;
+  }();
+#pragma unroll 3
+  for (int r = first; r < past; ++r) {
+    const double* const x = (r < a ? A + (long long)r * sa : B + (long long)(r - a) * sb) + p0;
+    int m = 0;
+    double v[EU];
+#pragma unroll
+    for (int u = 0; u < EU; ++u) v[u] = __ldg(x + off[u]);
+#pragma unroll
+    for (int u = 0; u < EU; ++u) {
+      const int e = biased_exponent(v[u]);
+      // |w| < 2^(ew - 1022), |b| < 2^(eb - 1022): the product's biased exponent is at most ew + eb - 1022
+      m = max(m, r < a || !w ? e : (e == 0x7ff ? e : max(e, 1) + ew[u]));
+    }
+    if (r >= a && w && wbad) m = 0x7ff;
+    m = __reduce_max_sync(0xffffffffu, min(m, 0x7ff));
+    if ((threadIdx.x & 31) == 0) atomicMax(top + (r - first), m);
+  }
+  __syncthreads();
+  if (threadIdx.x < past - first && top[threadIdx.x] > 0) atomicMax(emax + first + threadIdx.x, top[threadIdx.x]);
+}
+
+constexpr int GW = 4, GNT = 3;             // warps per CTA; 8-column tiles per warp
+constexpr int GROWS = 16 + 8 * GNT + 1;    // staged rows of a warp: A, B, w
+constexpr int GPITCH = 36;                 // doubles per staged row of 32 points (conflict-free fragment loads)
+constexpr size_t GSMEM = (size_t)GW * 2 * GROWS * GPITCH * sizeof(double);
+
+// One warp: 16 rows of A (blockIdx.y) by 24 columns of B (blockIdx.z) over windows of 32 points,
+// the next window's values on their way by cp.async (8-byte copies: any alignment) while this one
+// is split and multiplied.  Fragment k indices are points in an order that keeps a thread's
+// loads on four neighbouring points.
+__global__ void __launch_bounds__(32 * GW, 2)
+    gram64_kernel(long long n, int a, const double* __restrict__ A, long long sa, int b, const double* __restrict__ B,
+                  long long sb, const double* __restrict__ w, const int* __restrict__ emax, int sym,
+                  longlong2* __restrict__ part) {
+  const int i0 = blockIdx.y * 16, j0 = blockIdx.z * 8 * GNT;
+  if (sym && j0 + 8 * GNT <= i0) return;  // below the diagonal: mirrored by the reduction
+  extern __shared__ __align__(16) double gsm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  double* const st0 = gsm + (size_t)warp * 2 * GROWS * GPITCH;
+  const int na = min(16, a - i0), nb = min(8 * GNT, b - j0);
+  for (int e = lane; e < 2 * GROWS * GPITCH; e += 32) st0[e] = 0.0;  // rows past the operands stay zero
+  __syncwarp();
+  auto copy = [&](long long p0, int q) {
+    double* const d = st0 + q * GROWS * GPITCH + lane;
+    const long long p = p0 + lane;
+    const bool in = p < n;
+    const long long pc = in ? p : 0;
+    for (int r = 0; r < na; ++r) cp_async_zfill<8>(d + r * GPITCH, A + (long long)(i0 + r) * sa + pc, in);
+    for (int r = 0; r < nb; ++r) cp_async_zfill<8>(d + (16 + r) * GPITCH, B + (long long)(j0 + r) * sb + pc, in);
+    if (w) cp_async_zfill<8>(d + (GROWS - 1) * GPITCH, w + pc, in);
+  };
+  const int r0 = i0 + g, r1 = i0 + g + 8;
+  const int ea0 = r0 < a ? max(emax[r0], 1) : 1, ea1 = r1 < a ? max(emax[r1], 1) : 1;
+  int eb[GNT];
+#pragma unroll
+  for (int q = 0; q < GNT; ++q) {
+    const int j = j0 + 8 * q + g;
+    eb[q] = j < b ? max(emax[a + j], 1) : 1;
+  }
+  int s[GNT][4][SL];
+#pragma unroll
+  for (int q = 0; q < GNT; ++q)
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int l = 0; l < SL; ++l) s[q][c][l] = 0;
+  const long long step = (long long)gridDim.x * GW * 32;
+  long long p0 = ((long long)blockIdx.x * GW + warp) * 32;
+  if (p0 < n) copy(p0, 0);
+  cp_async_commit();
+  for (int buf = 0; p0 < n; p0 += step, buf ^= 1) {
+    if (p0 + step < n) copy(p0 + step, buf ^ 1);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncwarp();
+    const double* const sd = st0 + buf * GROWS * GPITCH + t;
+    uint32_t fa[2][4][SL];  // A fragments of both 16-point halves
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const double *x0 = sd + g * GPITCH + 16 * h, *x1 = x0 + 8 * GPITCH;
+      digits2(fixed63(x0[0], ea0), fixed63(x0[4], ea0), fa[h][0]);
+      digits2(fixed63(x1[0], ea1), fixed63(x1[4], ea1), fa[h][1]);
+      digits2(fixed63(x0[8], ea0), fixed63(x0[12], ea0), fa[h][2]);
+      digits2(fixed63(x1[8], ea1), fixed63(x1[12], ea1), fa[h][3]);
+    }
+#pragma unroll
+    for (int q = 0; q < GNT; ++q) {
+      if (j0 + 8 * q >= b) break;  // uniform
+      float acc[SL][4];
+#pragma unroll
+      for (int l = 0; l < SL; ++l)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[l][c] = 0.f;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double *xb = sd + (16 + 8 * q + g) * GPITCH + 16 * h, *xw = sd + (GROWS - 1) * GPITCH + 16 * h;
+        double x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = w ? xb[4 * k] * xw[4 * k] : xb[4 * k];
+        uint32_t b0[SL], b1[SL];
+        digits2(fixed63(x[0], eb[q]), fixed63(x[1], eb[q]), b0);
+        digits2(fixed63(x[2], eb[q]), fixed63(x[3], eb[q]), b1);
+        // consecutive products go to different levels (independent accumulators)
+#pragma unroll
+        for (int i = 0; i < SL; ++i)
+#pragma unroll
+          for (int j = 0; j < SL - i; ++j)
+            mma16816(acc[i + j], fa[h][0][i], fa[h][1][i], fa[h][2][i], fa[h][3][i], b0[j], b1[j]);
+        // the next level, scaled into the last one (2^-9 of a unit is exact in FP16; the accumulator may round
+        // below one unit here)
+        const __half2 sc = __half2half2(__float2half(1.f / 512.f));
+#pragma unroll
+        for (int j = 1; j < SL; ++j) {
+          const __half2 v0 = __hmul2(*reinterpret_cast<const __half2*>(&b0[j]), sc);
+          const __half2 v1 = __hmul2(*reinterpret_cast<const __half2*>(&b1[j]), sc);
+          mma16816(acc[SL - 1], fa[h][0][SL - j], fa[h][1][SL - j], fa[h][2][SL - j], fa[h][3][SL - j],
+                   *reinterpret_cast<const uint32_t*>(&v0), *reinterpret_cast<const uint32_t*>(&v1));
+        }
+      }
+#pragma unroll
+      for (int l = 0; l < SL; ++l)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s[q][c][l] += __float2int_rn(acc[l][c]);
+    }
+    __syncwarp();  // this buffer is refilled by the next window's copies
+  }
+  // integer sums of the warps of this CTA, one partial per CTA: every sum up to the output is exact
+  longlong2 (*const red)[16][8 * GNT] = reinterpret_cast<longlong2 (*)[16][8 * GNT]>(gsm);
+  cp_async_wait<0>();
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < GNT; ++q)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) red[warp][g + (c >= 2 ? 8 : 0)][8 * q + 2 * t + (c & 1)] = halves(s[q][c]);
+  __syncthreads();
+  longlong2* const pb = part + (long long)blockIdx.x * a * b;
+  for (int e = threadIdx.x; e < 16 * 8 * GNT; e += 32 * GW) {
+    const int i = e / (8 * GNT), j = e - i * (8 * GNT);
+    if (i0 + i < a && j0 + j < b) {
+      longlong2 v = make_longlong2(0, 0);
+#pragma unroll
+      for (int q = 0; q < GW; ++q) {
+        v.x += red[q][i][j].x;
+        v.y += red[q][i][j].y;
+      }
+      pb[(long long)(i0 + i) * b + j0 + j] = v;
+    }
+  }
+}
+
+// out[i][j] (+)= sum over CTAs, one warp per output; a symmetric product takes its lower triangle
+// from the upper.  Outputs whose row or column holds an infinity or a NaN (or may overflow) are
+// summed plainly in FP64 here.
+__global__ void gram64_reduce_kernel(int nblocks, long long n, int a, const double* __restrict__ A, long long sa, int b,
+                                     const double* __restrict__ B, long long sb, const double* __restrict__ w,
+                                     const int* __restrict__ emax, int sym, const longlong2* __restrict__ part,
+                                     double* __restrict__ out, int accumulate) {
+  const int lane = threadIdx.x & 31;
+  const long long ab = (long long)a * b;
+  for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < ab; e += (gridDim.x * blockDim.x) >> 5) {
+    const int i = e / b, j = e - i * b;
+    double v = 0.0;
+    if (emax[i] >= 0x7ff || emax[a + j] >= 0x7ff) {
+      for (long long p = lane; p < n; p += 32)
+        v += A[(long long)i * sa + p] * (B[(long long)j * sb + p] * (w ? w[p] : 1.0));
+    } else {
+      const long long at = sym && i > j ? (long long)j * b + i : e;
+      longlong2 q = make_longlong2(0, 0);
+      for (int k = lane; k < nblocks; k += 32) {
+        const longlong2 x = part[(long long)k * ab + at];
+        q.x += x.x;
+        q.y += x.y;
+      }
+      for (int off = 16; off > 0; off >>= 1) {
+        q.x += __shfl_down_sync(0xffffffffu, q.x, off);
+        q.y += __shfl_down_sync(0xffffffffu, q.y, off);
+      }
+      // a value of row r is its integer times 2^(emax - 1022 - 61); units 512^(12 - 5)
+      if (lane == 0) {
+        const int ei = max(sym && i > j ? emax[j] : emax[i], 1), ej = max(sym && i > j ? emax[a + i] : emax[a + j], 1);
+        v = join(q.x, q.y, ei + ej - 2166 + 63);
+      }
+    }
+    if (emax[i] >= 0x7ff || emax[a + j] >= 0x7ff)
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) out[e] = accumulate ? out[e] + v : v;
+  }
+}
+
+}  // namespace
+
+// Windows per warp stay below 120 (an int32 level sum takes 127 windows of at most 2^24).
+int gram64_split_launch(long long n, int a, const double* A, long long sa, int b, const double* B, long long sb,
+                        const double* w, double* out, int accumulate, longlong2* part, int max_blocks, int* emax,
+                        cudaStream_t st) {
+  const int sms = device_sm_count();
+  const int ty = (a + 15) / 16, tz = (b + 8 * GNT - 1) / (8 * GNT);
+  const long long windows = (n + 32 * GW - 1) / (32 * GW);
+  long long grid = std::min<long long>(windows, std::max(1, 2 * sms / (ty * tz)));
+  grid = std::min<long long>(std::max(grid, (windows + 119) / 120), max_blocks);
+  if (windows > 120 * grid) return -1;
+  const int sym = A == B && sa == sb && a == b;
+  if (cudaMemsetAsync(emax, 0, sizeof(int) * (a + b), st) != cudaSuccess) return IGD_ERR_CUDA;
+  row_exponent_kernel<<<dim3((unsigned)((n + ETH * EU - 1) / (ETH * EU)), (a + b + ER - 1) / ER), ETH, 0, st>>>(
+      n, a, A, sa, b, B, sb, w, emax);
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(gram64_kernel), GSMEM) != IGD_OK) return IGD_ERR_CUDA;
+  gram64_kernel<<<dim3((unsigned)grid, ty, tz), 32 * GW, GSMEM, st>>>(n, a, A, sa, b, B, sb, w, emax, sym, part);
+  gram64_reduce_kernel<<<std::min((a * b * 32 + 255) / 256, 1024), 256, 0, st>>>((int)grid, n, a, A, sa, b, B, sb, w,
+                                                                               emax, sym, part, out, accumulate);
+  return launch_status();
+}
+
+}  // namespace igd
