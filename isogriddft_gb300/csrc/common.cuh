@@ -115,6 +115,12 @@ int hpsi_agrid_lin_launch(int dtype, int closure, int nx, int ny, int nz, const 
                           const void* psi, void* out, int nb, long long ostride, double kscale, double vscale,
                           cudaStream_t st);
 
+// The linear-tile kernel as the Poisson operator of a Krylov solve, as hpsi_agrid_krylov below, in FP32 or
+// FP64 (acc[1] only when dot_y is null); -1 = not applicable.
+bool hpsi_agrid_lin_krylov_applies(int nx, int ny, int nz);
+int hpsi_agrid_lin_krylov(int dtype, int nx, int ny, int nz, const void* coeffs, const void* psi, void* out,
+                          double kscale, const void* dot_y, double* dot_acc, const int* skip, cudaStream_t st);
+
 // Whole-row z-vectorised fast path of igd_hpsi_agrid (hpsi_agrid_zvec.cu); -1 = not applicable.
 int hpsi_agrid_zvec_launch(int dtype, int closure, int nx, int ny, int nz, const void* coeffs, const void* veff,
                            const void* psi, void* out, int nb, long long ostride, double kscale, double vscale,

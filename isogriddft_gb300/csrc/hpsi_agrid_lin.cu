@@ -825,4 +825,23 @@ int hpsi_agrid_lin_launch(int dtype, int closure, int nx, int ny, int nz, const 
   return -1;
 }
 
+// lin_ok's rows split into tiles of two rows or more for every ny >= 3, so an applicable grid always has a plan.
+bool hpsi_agrid_lin_krylov_applies(int nx, int ny, int nz) { return lin_ok(nx, ny, nz); }
+
+int hpsi_agrid_lin_krylov(int dtype, int nx, int ny, int nz, const void* coeffs, const void* psi, void* out,
+                          double kscale, const void* dot_y, double* dot_acc, const int* skip, cudaStream_t st) {
+  if (!lin_ok(nx, ny, nz) || !dot_acc) return -1;
+  const long long n = (long long)nx * ny * nz;
+  if (dtype == IGD_F64)
+    return lin64_launch<true, true, false>(static_cast<const double*>(coeffs), nullptr, static_cast<const double*>(psi),
+                                           static_cast<double*>(out), nx, ny, nz, 1, n, kscale, st,
+                                           static_cast<const double*>(dot_y), dot_acc, skip);
+  const float *c = static_cast<const float*>(coeffs), *p = static_cast<const float*>(psi),
+              *y = static_cast<const float*>(dot_y);
+  float* o = static_cast<float*>(out);
+  if (nz > L32_NT * 2 / 5)
+    return lin32_launch<1, 3, true, true>(c, nullptr, p, o, nx, ny, nz, 1, n, kscale, 0.0, st, y, dot_acc, skip);
+  return lin32_launch<1, 2, true, true>(c, nullptr, p, o, nx, ny, nz, 1, n, kscale, 0.0, st, y, dot_acc, skip);
+}
+
 }  // namespace igd

@@ -515,16 +515,17 @@ int bicgstab(const Problem& P, const T* f, T* x, double rtol, int maxit, unsigne
   return h.status == IGD_ERR_NOT_CONVERGED ? IGD_OK : h.status;  // non-convergence is reported via rel
 }
 
-// ---- Fused FP32 BiCGSTAB for the monitor-grid operator of the whole-row
-// kernel (hpsi_agrid_krylov): the operator writes zero faces and returns the
-// dot products r^.v, t.s and t.t from its epilogue, so every vector keeps zero
+// ---- Fused BiCGSTAB for the monitor-grid operators with a Krylov mode (FP32: the whole-row and
+// the linear-tile kernel, FP64: the linear-tile kernel): the operator writes zero faces and
+// returns the dot products r^.v, t.s and t.t from its epilogue, so every vector keeps zero
 // faces without masks, and the scalars alpha, beta, omega and the stopping
 // test are recomputed by the vector kernels from rotating banks of sums:
 // iteration j of a chunk accumulates into bank j % 4, reads banks j-1 and j-2,
 // and its first kernel clears bank j+1 (chunks are a multiple of 4 long).
 // Per iteration: p update, v = A p (+ r^.v), s update, t = A s (+ t.s, t.t),
 // x / r update (+ r.r, r^.r): five launches, no single-thread kernels.
-// The arithmetic is the same BiCGSTAB as bicgstab<T> above.
+// The arithmetic is the same BiCGSTAB as bicgstab<T> above.  Vectors move in 16-byte pieces where
+// n and the pointers allow (E values), else value by value (odd grids).
 enum { B_RV = 0, B_VV = 1, B_TS = 2, B_TT = 3, B_RR = 4, B_RHR = 5, B_N = 6 };
 struct FState {
   double bnorm2;
@@ -533,27 +534,47 @@ struct FState {
 };
 static_assert(sizeof(FState) <= 256, "FState must fit the 256-byte state slot of the Krylov workspace");
 
+template <typename T, int E>
+__device__ __forceinline__ void fld(const T* __restrict__ p, long long v, T (&o)[E]) {
+  if constexpr (E == 1)
+    o[0] = p[v];
+  else
+    ldv<T>(p, v, o);
+}
+template <typename T, int E>
+__device__ __forceinline__ void fst(T* __restrict__ p, long long v, const T (&o)[E]) {
+  if constexpr (E == 1)
+    p[v] = o[0];
+  else
+    stv<T>(p, v, o);
+}
+
 __global__ void kf_state_init(FState* s) { memset(s, 0, sizeof(FState)); }
 
 // r = rhat = f (faces zero), x = p = v = 0; bnorm2 = ||f||^2
-__global__ void kf_init(long long nv, int nx, int ny, int nz, const float* __restrict__ f, float* x, float* r,
-                        float* rh, float* p, float* v, FState* s) {
-  float a = 0.f;
+template <typename T, int E>
+__global__ void kf_init(long long nv, int nx, int ny, int nz, const T* __restrict__ f, T* x, T* r, T* rh, T* p, T* v,
+                        FState* s) {
+  T a = T(0);
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nv; q += (long long)gridDim.x * blockDim.x) {
-    float ff[4];
-    ldv<float>(f, q, ff);
-    const unsigned fb = face_bits<4>(q, nx, ny, nz);
+    T ff[E], z[E];
+    fld<T, E>(f, q, ff);
+    unsigned fb;
+    if constexpr (E == 1)
+      fb = on_face(q, nx, ny, nz);
+    else
+      fb = face_bits<E>(q, nx, ny, nz);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      ff[e] = (fb >> e) & 1u ? 0.f : ff[e];
+    for (int e = 0; e < E; ++e) {
+      ff[e] = (fb >> e) & 1u ? T(0) : ff[e];
+      z[e] = T(0);
       a += ff[e] * ff[e];
     }
-    const float z[4] = {0.f, 0.f, 0.f, 0.f};
-    stv<float>(r, q, ff);
-    stv<float>(rh, q, ff);
-    stv<float>(x, q, z);
-    stv<float>(p, q, z);
-    stv<float>(v, q, z);
+    fst<T, E>(r, q, ff);
+    fst<T, E>(rh, q, ff);
+    fst<T, E>(x, q, z);
+    fst<T, E>(p, q, z);
+    fst<T, E>(v, q, z);
   }
   acc_add(&s->bnorm2, (double)a);
 }
@@ -583,15 +604,15 @@ __device__ __forceinline__ void f_stop(FState* s, int j, int status) {
 // Iteration j, part 1: the stopping test on the previous iteration (k_next of
 // bicgstab<T>), then p = r + beta (p - omega v), beta = (rho_k / rho_{k-1})
 // (alpha_{k-1} / omega_{k-1}) (p = r on the first iteration); clears bank j+1.
-__global__ void kf_p(long long nv, const float* __restrict__ r, float* __restrict__ p, const float* __restrict__ v,
-                     FState* s, int j, double rtol2, int maxit) {
+template <typename T, int E>
+__global__ void kf_p(long long nv, const T* __restrict__ r, T* __restrict__ p, const T* __restrict__ v, FState* s, int j, double rtol2, int maxit) {
   // the scalar work (FP64 divisions, slow on GB300's FP64 pipe) once per block;
   // stop: -1 go on, -2 stopped before, else the status this iteration stops with
-  __shared__ float sc[2];
+  __shared__ T sc[2];
   __shared__ int stop;
   if (threadIdx.x == 0) {
     int st = -1;
-    float bt = 0.f, om = 0.f;
+    T bt = T(0), om = T(0);
     if (s->done) {
       st = -2;
     } else {
@@ -608,8 +629,8 @@ __global__ void kf_p(long long nv, const float* __restrict__ r, float* __restric
           const double rho = b1[B_RHR], rho_prev = b2[B_RHR];
           const double alpha = rho_prev / b1[B_RV], omega = b1[B_TS] / b1[B_TT];
           if (!(fabs(rho) > 1e-300) || omega == 0.0) st = IGD_ERR_BREAKDOWN;
-          bt = (float)((rho / rho_prev) * (alpha / omega));
-          om = (float)omega;
+          bt = (T)((rho / rho_prev) * (alpha / omega));
+          om = (T)omega;
         }
         if (st < 0 && k >= maxit) st = IGD_ERR_NOT_CONVERGED;
       }
@@ -621,23 +642,24 @@ __global__ void kf_p(long long nv, const float* __restrict__ r, float* __restric
   }
   __syncthreads();
   if (stop != -1) return;
-  const float bt = sc[0], om = sc[1];
+  const T bt = sc[0], om = sc[1];
   if (blockIdx.x == 0 && threadIdx.x < B_N) s->bank[(j + 1) & 3][threadIdx.x] = 0.0;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nv; q += (long long)gridDim.x * blockDim.x) {
-    float rr4[4], pp[4], vv[4];
-    ldv<float>(r, q, rr4);
-    ldv<float>(p, q, pp);
-    ldv<float>(v, q, vv);
+    T rr4[E], pp[E], vv[E];
+    fld<T, E>(r, q, rr4);
+    fld<T, E>(p, q, pp);
+    fld<T, E>(v, q, vv);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) pp[e] = rr4[e] + bt * (pp[e] - om * vv[e]);
-    stv<float>(p, q, pp);
+    for (int e = 0; e < E; ++e) pp[e] = rr4[e] + bt * (pp[e] - om * vv[e]);
+    fst<T, E>(p, q, pp);
   }
 }
 
 // Part 2 (after v = A p and r^.v): alpha = rho_k / r^.v; s = r - alpha v.
-__global__ void kf_s(long long nv, const float* __restrict__ r, const float* __restrict__ v, float* __restrict__ sv,
-                     FState* s, int j) {
-  __shared__ float sal;
+template <typename T, int E>
+__global__ void kf_s(long long nv, const T* __restrict__ r, const T* __restrict__ v, T* __restrict__ sv, FState* s,
+                     int j) {
+  __shared__ T sal;
   __shared__ int go;
   if (threadIdx.x == 0) {
     go = 0;
@@ -646,31 +668,31 @@ __global__ void kf_s(long long nv, const float* __restrict__ r, const float* __r
       if (!(fabs(rv) > 1e-300) || !isfinite(rv)) {
         f_stop(s, j, IGD_ERR_BREAKDOWN);
       } else {
-        sal = (float)(s->bank[(j + 3) & 3][B_RHR] / rv);
+        sal = (T)(s->bank[(j + 3) & 3][B_RHR] / rv);
         go = 1;
       }
     }
   }
   __syncthreads();
   if (!go) return;
-  const float al = sal;
+  const T al = sal;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nv; q += (long long)gridDim.x * blockDim.x) {
-    float rr4[4], vv[4], o[4];
-    ldv<float>(r, q, rr4);
-    ldv<float>(v, q, vv);
+    T rr4[E], vv[E], o[E];
+    fld<T, E>(r, q, rr4);
+    fld<T, E>(v, q, vv);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) o[e] = rr4[e] - al * vv[e];
-    stv<float>(sv, q, o);
+    for (int e = 0; e < E; ++e) o[e] = rr4[e] - al * vv[e];
+    fst<T, E>(sv, q, o);
   }
 }
 
 // Part 3 (after t = A s, t.s, t.t): omega = t.s / t.t; x += alpha p + omega s;
 // r = s - omega t; r.r and r^.r into bank j.
-__global__ void kf_xr(long long nv, float* __restrict__ x, float* __restrict__ r, const float* __restrict__ p,
-                      const float* __restrict__ sv, const float* __restrict__ t, const float* __restrict__ rh,
-                      FState* s, int j) {
+template <typename T, int E>
+__global__ void kf_xr(long long nv, T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
+                      const T* __restrict__ sv, const T* __restrict__ t, const T* __restrict__ rh, FState* s, int j) {
   double* b0 = s->bank[j & 3];
-  __shared__ float sc[2];
+  __shared__ T sc[2];
   __shared__ int go;
   if (threadIdx.x == 0) {
     go = 0;
@@ -679,58 +701,79 @@ __global__ void kf_xr(long long nv, float* __restrict__ x, float* __restrict__ r
       if (!(tt > 0.0) || !isfinite(tt)) {
         f_stop(s, j, IGD_ERR_BREAKDOWN);
       } else {
-        sc[0] = (float)(s->bank[(j + 3) & 3][B_RHR] / b0[B_RV]);
-        sc[1] = (float)(b0[B_TS] / tt);
+        sc[0] = (T)(s->bank[(j + 3) & 3][B_RHR] / b0[B_RV]);
+        sc[1] = (T)(b0[B_TS] / tt);
         go = 1;
       }
     }
   }
   __syncthreads();
   if (!go) return;
-  const float al = sc[0], om = sc[1];
-  float a = 0.f, b = 0.f;
+  const T al = sc[0], om = sc[1];
+  T a = T(0), b = T(0);
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nv; q += (long long)gridDim.x * blockDim.x) {
-    float xx[4], pp[4], ss[4], tv[4], hh[4], ro[4];
-    ldv<float>(x, q, xx);
-    ldv<float>(p, q, pp);
-    ldv<float>(sv, q, ss);
-    ldv<float>(t, q, tv);
-    ldv<float>(rh, q, hh);
+    T xx[E], pp[E], ss[E], tv[E], hh[E], ro[E];
+    fld<T, E>(x, q, xx);
+    fld<T, E>(p, q, pp);
+    fld<T, E>(sv, q, ss);
+    fld<T, E>(t, q, tv);
+    fld<T, E>(rh, q, hh);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
+    for (int e = 0; e < E; ++e) {
       xx[e] = xx[e] + al * pp[e] + om * ss[e];
       ro[e] = ss[e] - om * tv[e];
       a += ro[e] * ro[e];
       b += hh[e] * ro[e];
     }
-    stv<float>(x, q, xx);
-    stv<float>(r, q, ro);
+    fst<T, E>(x, q, xx);
+    fst<T, E>(r, q, ro);
   }
   acc_add2(&b0[B_RR], (double)a, &b0[B_RHR], (double)b);
 }
 
-// igd_poisson_select: 0 = the fused FP32 path wherever it applies, 1 = never (per host thread).
+// igd_poisson_select: 0 = the fused path wherever it applies, 1 = never (per host thread).
 thread_local int g_poisson_path = 0;
 bool fused_poisson_enabled() { return g_poisson_path == 0; }
 
-// The fused path applies: monitor grid, FP32 whole-row operator, 16-byte vectors.
-bool fused_applies(const Problem& P, const void* a, const void* b, const void* ws) {
-  const auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
-  return P.kind == IGD_GRID_MONITOR && P.c32 && hpsi_agrid_krylov_applies(P.nz, P.c32) && P.n % 4 == 0 && al16(a) &&
-         al16(b) && al16(ws);
+// The operator of the fused path: out = -L psi with the dots (see hpsi_agrid_krylov), -1 when neither
+// kernel takes it.  Where both FP32 kernels do, small grids go to the linear-tile kernel: the
+// whole-row kernel's march has a latency of 14 us (27 us with rows of more than 128 points), whole-row
+// / linear-tile 48^3 14.3 / 8.1 us, 80^3 14.6 / 11.5, 68x84x92 14.8 / 12.6, 96^3 14.7 / 15.5, 128^3
+// 18.3 / 28.8; 64x64x192 27 / 17, 128x128x192 38 / 68.
+template <typename T>
+int krylov_op(const Problem& P, const T* psi, T* out, const T* dot_y, double* acc, const int* skip, cudaStream_t q) {
+  if constexpr (sizeof(T) == 4) {
+    const float* c = static_cast<const float*>(P.c32);
+    const bool small = P.n <= (P.nz <= 128 ? 600000 : 1200000) && hpsi_agrid_lin_krylov_applies(P.nx, P.ny, P.nz);
+    if (!small && hpsi_agrid_krylov_applies(P.nz, c)) {
+      const int e = hpsi_agrid_krylov(P.nx, P.ny, P.nz, c, psi, out, -1.0, dot_y, acc, skip, q);
+      if (e != -1) return e;
+    }
+    return hpsi_agrid_lin_krylov(IGD_F32, P.nx, P.ny, P.nz, c, psi, out, -1.0, dot_y, acc, skip, q);
+  } else {
+    return hpsi_agrid_lin_krylov(IGD_F64, P.nx, P.ny, P.nz, P.c64, psi, out, -1.0, dot_y, acc, skip, q);
+  }
 }
 
-int bicgstab_fused(const Problem& P, const float* f, float* x, double rtol, int maxit, unsigned char* ws, int* iters,
-                   double* rel) {
-  const long long n = P.n, nv = n / 4;
-  float* r = reinterpret_cast<float*>(ws);
-  float *rh = r + n, *p = rh + n, *v = p + n, *sv = v + n, *t = sv + n;
-  FState* S = reinterpret_cast<FState*>(ws + 6 * (size_t)n * sizeof(float));
-  const float* c32 = static_cast<const float*>(P.c32);
+// The fused path applies: a monitor grid whose rows a Krylov-mode operator takes.
+template <typename T>
+bool fused_applies(const Problem& P) {
+  if (P.kind != IGD_GRID_MONITOR || (sizeof(T) == 4 && !P.c32)) return false;
+  if (sizeof(T) == 4 && hpsi_agrid_krylov_applies(P.nz, P.c32)) return true;
+  return hpsi_agrid_lin_krylov_applies(P.nx, P.ny, P.nz);
+}
+
+template <typename T, int E>
+int bicgstab_fused_run(const Problem& P, const T* f, T* x, double rtol, int maxit, unsigned char* ws, int* iters,
+                       double* rel, double* bnorm) {
+  const long long n = P.n, nv = n / E;
+  T* r = reinterpret_cast<T*>(ws);
+  T *rh = r + n, *p = rh + n, *v = p + n, *sv = v + n, *t = sv + n;
+  FState* S = reinterpret_cast<FState*>(ws + 6 * (size_t)n * sizeof(T));
   const int nbv = pblocks(nv);
   cudaStream_t st = P.st;
   kf_state_init<<<1, 1, 0, st>>>(S);
-  kf_init<<<nbv, PB, 0, st>>>(nv, P.nx, P.ny, P.nz, f, x, r, rh, p, v, S);
+  kf_init<T, E><<<nbv, PB, 0, st>>>(nv, P.nx, P.ny, P.nz, f, x, r, rh, p, v, S);
   kf_after_init<<<1, 1, 0, st>>>(S);
   const double rtol2 = rtol * rtol;
   constexpr int chunk = 8;  // a multiple of the 4 banks
@@ -738,13 +781,13 @@ int bicgstab_fused(const Problem& P, const float* f, float* x, double rtol, int 
     kf_chunk_begin<<<1, 1, 0, q>>>(S, chunk);
     for (int j = 0; j < chunk; ++j) {
       double* bank = S->bank[j & 3];
-      kf_p<<<nbv, PB, 0, q>>>(nv, r, p, v, S, j, rtol2, maxit);
-      int e = hpsi_agrid_krylov(P.nx, P.ny, P.nz, c32, p, v, -1.0, rh, bank + B_RV, &S->done, q);
+      kf_p<T, E><<<nbv, PB, 0, q>>>(nv, r, p, v, S, j, rtol2, maxit);
+      int e = krylov_op<T>(P, p, v, rh, bank + B_RV, &S->done, q);
       if (e) return e < 0 ? IGD_ERR_ARG : e;
-      kf_s<<<nbv, PB, 0, q>>>(nv, r, v, sv, S, j);
-      e = hpsi_agrid_krylov(P.nx, P.ny, P.nz, c32, sv, t, -1.0, nullptr, bank + B_TS, &S->done, q);
+      kf_s<T, E><<<nbv, PB, 0, q>>>(nv, r, v, sv, S, j);
+      e = krylov_op<T>(P, sv, t, nullptr, bank + B_TS, &S->done, q);
       if (e) return e < 0 ? IGD_ERR_ARG : e;
-      kf_xr<<<nbv, PB, 0, q>>>(nv, x, r, p, sv, t, rh, S, j);
+      kf_xr<T, E><<<nbv, PB, 0, q>>>(nv, x, r, p, sv, t, rh, S, j);
     }
     return launch_status();
   };
@@ -788,7 +831,19 @@ int bicgstab_fused(const Problem& P, const float* f, float* x, double rtol, int 
   *iters = h.done ? h.base + h.stop : std::min(launched, maxit);
   const double rr = h.done ? h.bank[(h.stop + 3) & 3][B_RR] : h.bank[(chunk - 1) & 3][B_RR];
   *rel = h.bnorm2 > 0 ? std::sqrt(rr / h.bnorm2) : 0.0;
+  if (bnorm) *bnorm = std::sqrt(h.bnorm2);
   return h.status == IGD_ERR_NOT_CONVERGED ? IGD_OK : h.status;  // non-convergence is reported via rel
+}
+
+// Pieces of 16 bytes when they neither cross a grid row nor break the alignment of any vector.
+template <typename T>
+int bicgstab_fused(const Problem& P, const T* f, T* x, double rtol, int maxit, unsigned char* ws, int* iters,
+                   double* rel, double* bnorm = nullptr) {
+  constexpr int E = VecT<T>::E;
+  const auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+  if (P.nz % E == 0 && al16(f) && al16(x) && al16(ws))
+    return bicgstab_fused_run<T, E>(P, f, x, rtol, maxit, ws, iters, rel, bnorm);
+  return bicgstab_fused_run<T, 1>(P, f, x, rtol, maxit, ws, iters, rel, bnorm);
 }
 
 __global__ void k_zero_u64(unsigned long long* a, double* b) {
@@ -838,7 +893,7 @@ int true_residual(const Problem& P, const double* f, const double* u, double* Au
 
 using namespace igd;
 
-// Test hook: 0 = the fused FP32 BiCGSTAB (operator-epilogue dots, no scalar
+// Test hook: 0 = the fused BiCGSTAB (operator-epilogue dots, no scalar
 // kernels) wherever it applies, 1 = the unfused iteration; per host thread.
 extern "C" int igd_poisson_select(int path) {
   if (path < 0 || path > 1) return IGD_ERR_ARG;
@@ -873,8 +928,10 @@ static int poisson_solve(int grid_kind, int precision, int nx, int ny, int nz, c
   unsigned char* kry = w + 2 * (size_t)n * sizeof(double) + 256;
   int iters = 0, rounds = 0, status = IGD_OK;
   double rel = 0.0, rnorm = 0.0, rmax = 0.0, fnorm = 0.0;
+  const bool fused64 = precision == IGD_PREC_FP64 && fused_poisson_enabled() && fused_applies<double>(P);
   if (precision == IGD_PREC_FP64 && !from_u) {
-    status = bicgstab<double>(P, f, u, rtol, max_iterations, kry, &iters, &rel, &fnorm);
+    status = fused64 ? bicgstab_fused<double>(P, f, u, rtol, max_iterations, kry, &iters, &rel, &fnorm)
+                     : bicgstab<double>(P, f, u, rtol, max_iterations, kry, &iters, &rel, &fnorm);
     rounds = 1;
   } else if (precision == IGD_PREC_FP64) {
     // one correction solve A d = f - A u0 to rtol ||f|| / ||f - A u0||, then u = u0 + d
@@ -884,7 +941,8 @@ static int poisson_solve(int grid_kind, int precision, int nx, int ny, int nz, c
     if (e) return e;
     if (rnorm > rtol * fnorm) {
       double inner_rel = 0.0;
-      status = bicgstab<double>(P, res, Au, rtol * fnorm / rnorm, max_iterations, kry, &iters, &inner_rel);
+      status = fused64 ? bicgstab_fused<double>(P, res, Au, rtol * fnorm / rnorm, max_iterations, kry, &iters, &inner_rel)
+                       : bicgstab<double>(P, res, Au, rtol * fnorm / rnorm, max_iterations, kry, &iters, &inner_rel);
       k_add_masked<<<pblocks(n), PB, 0, P.st>>>(n, nx, ny, nz, u, Au);
       rounds = 1;
     }
@@ -892,7 +950,7 @@ static int poisson_solve(int grid_kind, int precision, int nx, int ny, int nz, c
     float* r32 = reinterpret_cast<float*>(kry);
     float* d32 = r32 + n;
     unsigned char* k32 = kry + 2 * (size_t)n * sizeof(float);
-    const bool fused = fused_poisson_enabled() && fused_applies(P, r32, d32, k32);
+    const bool fused = fused_poisson_enabled() && fused_applies<float>(P);
     int e;
     if (from_u) {
       e = rhs_norm(P, f, Au, res, scal, &fnorm);
@@ -910,7 +968,7 @@ static int poisson_solve(int grid_kind, int precision, int nx, int ny, int nz, c
       int it = 0;
       double inner_rel = 0.0;
       const double inner_tol = std::max(1e-5, 0.5 * rtol * fnorm / rnorm);
-      status = fused ? bicgstab_fused(P, r32, d32, inner_tol, max_iterations - iters, k32, &it, &inner_rel)
+      status = fused ? bicgstab_fused<float>(P, r32, d32, inner_tol, max_iterations - iters, k32, &it, &inner_rel)
                      : bicgstab<float>(P, r32, d32, inner_tol, max_iterations - iters, k32, &it, &inner_rel);
       iters += it;
       ++rounds;
