@@ -265,6 +265,14 @@ __global__ void gram_reduce_kernel(int nblocks, int ab, const double* __restrict
 }
 
 constexpr int RTH = 256;
+// FP32 rotations.  Two points per thread from ROT_PAIR_POINTS on: 21 rows to 20 columns take 8.4 us with
+// one and 7.4 with two over 117649 points; over 40000, 5.3 with one.
+constexpr long long ROT_PAIR_POINTS = 100000;
+// The pipeline's batches and its lower line: 22 rows to 20 columns over 363608 points take 15.2 us there and
+// 14.9 in the register kernel, 50 to 35 over 10^6 124 and 160, 19 to 12 23 and 37 (rotate_kernel).  Its
+// coefficients, rows x columns, have to leave room for two CTAs on an SM.
+constexpr int ROT_STAGES = 3, ROT_ROWS = 8;
+constexpr long long ROT_PIPE_POINTS = 1 << 19, ROT_PIPE_COEF = 6 * 1024;
 
 // out[j][p] (+)= sum_i A[i][p] C1[i][j] + sum_i B[i][p] C2[i][j] for j in
 // [j0, j0 + RC), RC from rotate_dispatch.
@@ -324,7 +332,6 @@ template <typename T, int RC>
 int rotate_launch(long long n, int a, const T* A, long long sa, const double* C1, int b, const T* B, long long sb,
                   const double* C2, int c, T* out, long long so, int accumulate, cudaStream_t st) {
   const size_t smem = (size_t)(a + b) * RC * sizeof(T);
-  if (smem > 200 * 1024) return IGD_ERR_TOO_LARGE;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(rotate_kernel<T, RC>), smem) != IGD_OK) return IGD_ERR_CUDA;
   const long long blocks = std::min<long long>((n + RTH - 1) / RTH, 152LL * 8);
   dim3 grid((unsigned)blocks, (c + RC - 1) / RC);
@@ -332,9 +339,270 @@ int rotate_launch(long long n, int a, const T* A, long long sa, const double* C1
   return IGD_OK;
 }
 
+// Two FP32 FMAs on a packed pair, each rounded as fmaf: same rate as two FMAs, half the issue slots.
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long x, unsigned long long c) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(x), "l"(c));
+}
+__device__ __forceinline__ unsigned long long dup2(float x) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+  return d;
+}
+__device__ __forceinline__ float lane_of(unsigned long long d, int odd) {
+  return __uint_as_float((unsigned)(odd ? d >> 32 : d));
+}
+
+// FP32 rotation with the rows straight from memory, for rows that the pipeline
+// cannot copy in 16-byte pieces and for small grids: PP points per thread, RTH
+// apart, so the loads are coalesced whatever the strides and the alignment, and
+// packed column pairs, up to the next multiple of four.  50 rows to 35 columns
+// over 1000003 points: rotate_kernel (two tiles of 32) 317 us, this form 160; 22 to
+// 20 over 363609: 26.8 and 15.8.
+template <int RC, int PP>
+__global__ void __launch_bounds__(RTH, RC * PP <= 20 ? 3 : 2) rotate32_kernel(long long n, int a, const float* __restrict__ A,
+                                                          long long sa, const double* __restrict__ C1, int b,
+                                                          const float* __restrict__ B, long long sb,
+                                                          const double* __restrict__ C2, int c,
+                                                          float* __restrict__ out, long long so, int accumulate) {
+  constexpr int U = PP == 2 && RC >= 24 ? (RC >= 32 ? 4 : 2) : 8;  // rows whose loads are in flight together
+  extern __shared__ __align__(16) unsigned char rsm[];
+  float* cs = reinterpret_cast<float*>(rsm);  // (a + b) x RC
+  const int j0 = blockIdx.y * RC;
+  const int nj = min(RC, c - j0);
+  for (int e = threadIdx.x; e < (a + b) * RC; e += RTH) {
+    const int i = e / RC, jj = e - i * RC;
+    double v = 0.0;
+    if (jj < nj) v = i < a ? C1[(long long)i * c + j0 + jj] : C2[(long long)(i - a) * c + j0 + jj];
+    cs[e] = float(v);
+  }
+  __syncthreads();
+  for (long long p0 = blockIdx.x * (long long)(RTH * PP) + threadIdx.x; p0 < n;
+       p0 += (long long)gridDim.x * (RTH * PP)) {
+    unsigned long long acc[PP][RC / 2];
+#pragma unroll
+    for (int q = 0; q < PP; ++q)
+#pragma unroll
+      for (int jj = 0; jj < RC / 2; ++jj) acc[q][jj] = 0ull;
+    bool in[PP];
+#pragma unroll
+    for (int q = 0; q < PP; ++q) in[q] = p0 + q * RTH < n;
+    auto rows = [&](const float* __restrict__ M, long long sm, int m, const float* coef) {
+      M += p0;
+      auto row_fma = [&](const float(&x)[PP], const float* row) {
+        unsigned long long xx[PP];
+#pragma unroll
+        for (int q = 0; q < PP; ++q) xx[q] = dup2(x[q]);
+#pragma unroll
+        for (int j4 = 0; j4 < RC / 4; ++j4) {
+          const ulonglong2 k = reinterpret_cast<const ulonglong2*>(row)[j4];
+#pragma unroll
+          for (int q = 0; q < PP; ++q) {
+            fma2(acc[q][2 * j4], xx[q], k.x);
+            fma2(acc[q][2 * j4 + 1], xx[q], k.y);
+          }
+        }
+      };
+      int i = 0;
+      for (; i + U <= m; i += U) {
+        float x[U][PP];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int q = 0; q < PP; ++q) x[u][q] = in[q] ? M[(long long)(i + u) * sm + q * RTH] : 0.f;
+#pragma unroll
+        for (int u = 0; u < U; ++u) row_fma(x[u], coef + (i + u) * RC);
+      }
+      for (; i < m; ++i) {
+        float x[PP];
+#pragma unroll
+        for (int q = 0; q < PP; ++q) x[q] = in[q] ? M[(long long)i * sm + q * RTH] : 0.f;
+        row_fma(x, coef + i * RC);
+      }
+    };
+    rows(A, sa, a, cs);
+    if (b) rows(B, sb, b, cs + a * RC);
+#pragma unroll
+    for (int q = 0; q < PP; ++q)
+      if (in[q]) {
+#pragma unroll
+        for (int jj = 0; jj < RC; ++jj)
+          if (jj < nj) {
+            float* o = out + (long long)(j0 + jj) * so + p0 + q * RTH;
+            const float v = lane_of(acc[q][jj / 2], jj & 1);
+            *o = accumulate ? *o + v : v;
+          }
+      }
+  }
+}
+
+template <int RC>
+int rotate32_launch(long long n, int a, const float* A, long long sa, const double* C1, int b, const float* B,
+                    long long sb, const double* C2, int c, float* out, long long so, int accumulate, cudaStream_t st) {
+  const size_t smem = (size_t)(a + b) * RC * sizeof(float);
+  auto go = [&](auto kern, int pp) {
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != IGD_OK) return IGD_ERR_CUDA;
+    const long long blocks = std::min<long long>((n + RTH * pp - 1) / (RTH * pp), 152LL * 8);
+    kern<<<dim3((unsigned)blocks, (c + RC - 1) / RC), RTH, smem, st>>>(n, a, A, sa, C1, b, B, sb, C2, c, out, so,
+                                                                       accumulate);
+    return IGD_OK;
+  };
+  if (n >= ROT_PAIR_POINTS) return go(rotate32_kernel<RC, 2>, 2);
+  return go(rotate32_kernel<RC, 1>, 1);
+}
+
+// FP32 rotation through a shared-memory pipeline: the sums of rotate_kernel in
+// the same order.  A CTA takes tiles of PT points and all H * CW output columns;
+// a thread takes Q groups of four consecutive points and CW columns, so a
+// 16-byte coefficient read serves 16 Q FMAs (one point per thread: four, and
+// the shared-memory port is the bound).  Rows arrive in batches of ROT_ROWS
+// through a ring of ROT_STAGES cp.async stages that runs on across tiles.
+// 47 rows to 32 columns over 192^3 points: rotate_kernel 1009 us, this form 549
+// (floor 329 at the memory, 285 at the FP32 pipe), with Q = 1 and CW = 16, whose
+// coefficient reads weigh more, 599; with one batch of 4 rows per stage 710.
+template <int Q, int CW, int H>
+__global__ void __launch_bounds__(RTH, Q * CW <= 16 ? 2 : 1)
+    rotate_pipe_kernel(long long n, int a, const float* __restrict__ A, long long sa, const double* __restrict__ C1,
+                       int b, const float* __restrict__ B, long long sb, const double* __restrict__ C2, int c,
+                       float* __restrict__ out, long long so, int accumulate) {
+  constexpr int TH = RTH / H, PT = 4 * Q * TH, W = H * CW;
+  extern __shared__ __align__(16) unsigned char rsm[];
+  float* xs = reinterpret_cast<float*>(rsm);    // ROT_STAGES x ROT_ROWS x PT
+  float* cs = xs + ROT_STAGES * ROT_ROWS * PT;  // (a + b) x W
+  const int j0 = blockIdx.y * W;
+  const int m = a + b, tid = threadIdx.x;
+  for (int e = tid; e < m * W; e += RTH) {
+    const int i = e / W, jj = e - i * W;
+    double v = 0.0;
+    if (j0 + jj < c) v = i < a ? C1[(long long)i * c + j0 + jj] : C2[(long long)(i - a) * c + j0 + jj];
+    cs[e] = float(v);
+  }
+  const int batches = (m + ROT_ROWS - 1) / ROT_ROWS;
+  const long long tiles = (n + PT - 1) / PT;
+  const long long mine = tiles > blockIdx.x ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  // tile and batch of the next stage to fetch, stages left
+  long long ft = blockIdx.x, left = mine * batches;
+  int fb = 0;
+  const unsigned xs0 = (unsigned)__cvta_generic_to_shared(xs);
+  auto fetch = [&](int slot) {
+    if (left > 0) {
+      --left;
+      constexpr int V = PT / 4;  // 16-byte pieces of a row; points past n read as zero
+      const long long p0 = ft * PT;
+      const int i0 = fb * ROT_ROWS, rows = min(ROT_ROWS, m - i0);
+      const int x = (tid % V) * 4;
+      const long long rest = n - p0 - x;
+      const int bytes = rest >= 4 ? 16 : rest > 0 ? (int)rest * 4 : 0;
+      for (int r = tid / V; r < rows; r += RTH / V) {
+        const int i = i0 + r;
+        const float* src = (i < a ? A + (long long)i * sa : B + (long long)(i - a) * sb) + (bytes ? p0 + x : 0);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                         xs0 + (unsigned)((slot * ROT_ROWS + r) * PT + x) * 4u),
+                     "l"(src), "r"(bytes)
+                     : "memory");
+      }
+      if (++fb == batches) {
+        fb = 0;
+        ft += gridDim.x;
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+#pragma unroll
+  for (int k = 0; k < ROT_STAGES - 1; ++k) fetch(k);
+
+  const int part = tid / TH, px = (tid % TH) * 4;
+  int slot = 0;
+  for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+    unsigned long long acc[4 * Q][CW / 2];
+#pragma unroll
+    for (int q = 0; q < 4 * Q; ++q)
+#pragma unroll
+      for (int jj = 0; jj < CW / 2; ++jj) acc[q][jj] = 0ull;
+    for (int ib = 0; ib < batches; ++ib) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(ROT_STAGES - 2) : "memory");
+      __syncthreads();  // the stage is visible, and every thread has left the one refilled next
+      fetch(slot == 0 ? ROT_STAGES - 1 : slot - 1);
+      const float* x0 = xs + slot * ROT_ROWS * PT + px;
+      const float* k0 = cs + ib * ROT_ROWS * W + part * CW;
+      const int rows = min(ROT_ROWS, m - ib * ROT_ROWS);
+      auto row = [&](int r) {
+        unsigned long long xx[4 * Q];
+#pragma unroll
+        for (int g = 0; g < Q; ++g) {
+          const float4 x = *reinterpret_cast<const float4*>(x0 + r * PT + g * 4 * TH);
+          xx[4 * g] = dup2(x.x);
+          xx[4 * g + 1] = dup2(x.y);
+          xx[4 * g + 2] = dup2(x.z);
+          xx[4 * g + 3] = dup2(x.w);
+        }
+#pragma unroll
+        for (int j4 = 0; j4 < CW / 4; ++j4) {
+          const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(k0 + r * W + 4 * j4);
+#pragma unroll
+          for (int q = 0; q < 4 * Q; ++q) {
+            fma2(acc[q][2 * j4], xx[q], k.x);
+            fma2(acc[q][2 * j4 + 1], xx[q], k.y);
+          }
+        }
+      };
+      if (rows == ROT_ROWS) {
+#pragma unroll 2  // four spill
+        for (int r = 0; r < ROT_ROWS; ++r) row(r);
+      } else {
+        for (int r = 0; r < rows; ++r) row(r);
+      }
+      slot = slot == ROT_STAGES - 1 ? 0 : slot + 1;
+    }
+#pragma unroll
+    for (int g = 0; g < Q; ++g) {
+      const long long p = t * PT + g * 4 * TH + px;
+#pragma unroll
+      for (int jj = 0; jj < CW; ++jj) {
+        const int j = j0 + part * CW + jj;
+        if (j >= c) continue;
+        float* o = out + (long long)j * so + p;
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = lane_of(acc[4 * g + q][jj / 2], jj & 1);
+        if (p + 4 <= n) {
+          float4* o4 = reinterpret_cast<float4*>(o);
+          if (accumulate) {
+            const float4 w = *o4;
+            *o4 = make_float4(w.x + v[0], w.y + v[1], w.z + v[2], w.w + v[3]);
+          } else {
+            *o4 = make_float4(v[0], v[1], v[2], v[3]);
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (p + q < n) o[q] = accumulate ? o[q] + v[q] : v[q];
+        }
+      }
+    }
+  }
+}
+
+template <int Q, int CW, int H>
+int rotate_pipe_launch(long long n, int a, const float* A, long long sa, const double* C1, int b, const float* B,
+                       long long sb, const double* C2, int c, float* out, long long so, int accumulate,
+                       cudaStream_t st) {
+  constexpr int PT = 4 * Q * RTH / H, W = H * CW;
+  const size_t smem = (size_t)ROT_STAGES * ROT_ROWS * PT * 4 + (size_t)(a + b) * W * 4;
+  auto kern = rotate_pipe_kernel<Q, CW, H>;
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != IGD_OK) return IGD_ERR_CUDA;
+  const long long blocks = std::min<long long>((n + PT - 1) / PT, (Q * CW <= 16 ? 2LL : 1LL) * device_sm_count());
+  kern<<<dim3((unsigned)blocks, (c + W - 1) / W), RTH, smem, st>>>(n, a, A, sa, C1, b, B, sb, C2, c, out, so,
+                                                                   accumulate);
+  return IGD_OK;
+}
+
 template <typename T>
 int rotate_dispatch(long long n, int a, const T* A, long long sa, const double* C1, int b, const T* B, long long sb,
                     const double* C2, int c, T* out, long long so, int accumulate, cudaStream_t st) {
+  // coefficients of one column tile in shared memory, by the padded widths of the plain kernel; every
+  // other form's tile is no larger
+  const int rc = c <= 4 ? 4 : c <= 8 ? 8 : c <= 16 ? 16 : 32;
+  if ((size_t)(a + b) * rc * sizeof(T) > 200 * 1024) return IGD_ERR_TOO_LARGE;
   if constexpr (sizeof(T) == 8) {
     // The FP64 pipe (two lanes per clock and SM) bounds this form, so no column is padded: equal
     // tiles of at most 20 columns (40 accumulator registers), the width compiled in.  21 -> 20
@@ -351,10 +619,35 @@ int rotate_dispatch(long long n, int a, const T* A, long long sa, const double* 
     }
     return IGD_ERR_ARG;
   } else {
+    const int cols = std::min(c, 64);
+    auto al = [](const void* p, long long s) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && s % 4 == 0; };
+    if (n >= ROT_PIPE_POINTS && (long long)(a + b) * cols <= ROT_PIPE_COEF && al(A, sa) && (b == 0 || al(B, sb)) &&
+        al(out, so)) {
+#define IGD_ROT(LO, Q, CW, HH) \
+  if (cols > LO) return rotate_pipe_launch<Q, CW, HH>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
+      IGD_ROT(48, 1, 16, 4)
+      IGD_ROT(32, 1, 12, 4)
+      IGD_ROT(24, 2, 8, 4)
+      IGD_ROT(16, 1, 12, 2)
+      IGD_ROT(12, 1, 16, 1)
+      IGD_ROT(8, 1, 12, 1)
+      IGD_ROT(4, 1, 8, 1)
+      IGD_ROT(0, 1, 4, 1)
+#undef IGD_ROT
+    }
+    // up to 16 columns the plain kernel's occupancy counts for more: 19 rows to 12 columns over 1000003
+    // points take 37.5 us there, 46 with packed pairs
     if (c <= 4) return rotate_launch<T, 4>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
     if (c <= 8) return rotate_launch<T, 8>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
     if (c <= 16) return rotate_launch<T, 16>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
-    return rotate_launch<T, 32>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
+    const int tiles = (c + 31) / 32;
+    switch (((c + tiles - 1) / tiles + 3) / 4) {
+#define IGD_ROT(Q) \
+  case Q: return rotate32_launch<4 * Q>(n, a, A, sa, C1, b, B, sb, C2, c, out, so, accumulate, st);
+      IGD_ROT(5) IGD_ROT(6) IGD_ROT(7) IGD_ROT(8)
+#undef IGD_ROT
+    }
+    return IGD_ERR_ARG;
   }
 }
 
