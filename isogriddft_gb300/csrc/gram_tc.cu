@@ -27,16 +27,29 @@
 // FP64 once per CTA and are summed in FP64 across blocks (deterministic
 // per-block partials reduced by gram_reduce_kernel).
 //
-// Roles (128 + NW threads, one CTA per SM, persistent over stages):
-//   warp 0 lane 0: TMA producer (FP32 tiles of A and B with 128-byte swizzle,
-//                  w by a 1-D tensor copy) into an S-slot ring;
-//   warp 1       : TMEM allocation; lane 0 issues the MMAs (12 per stage);
-//   warps 4..    : NW worker threads for the split pass (B *= w, hi in place,
-//                  lo to a second tile, proxy fence); warps 4-7 (one per TMEM
-//                  lane quarter) also run the epilogue (TMEM -> FP64 sums).
+// Roles (384 threads, one CTA per SM, persistent over stages):
+//   warp 0 lane 0: TMA producer (FP32 tiles of A and B with 128-byte swizzle)
+//                  into a ring of raw slots;
+//   warp 1       : TMEM allocation; lane 0 issues the MMAs (8 per stage: hi*hi and
+//                  hi*lo in one of twice the width, since B's lo tile follows its
+//                  hi tile, and lo*hi);
+//   warps 4-11   : two groups of four warps that take the stages in turn: raw slot
+//                  -> (B *= w) -> hi and lo tiles of the group's split buffer, proxy
+//                  fence.  Two per TMEM lane quarter, they also run the epilogue
+//                  (TMEM -> compensated sums), each for half of the columns.
+// The weights come straight from memory, one stage ahead, in the splitting
+// threads' registers: in the ring they would cost it its third slot.
 // Two TMEM accumulator pairs alternate between windows so MMAs continue while
 // the previous window is read out.  Every wait is bounded: on a timeout the error
 // word is set, all roles leave their loops, TMEM is freed.
+//
+// What bounds it: shared memory.  A stage of 128 rows moves 32 KB in by TMA, 32 KB
+// out and 64 KB back for the split and 80 KB to the tensor core, 0.9 us at 128 bytes
+// a clock; it takes 1.1.  One group that split in place in a raw slot took 1.3 for
+// narrow blocks and 1.7 for wide ones (four worker warps: the epilogue held all 64
+// columns of a row in one thread).  Over 192^3 points, before and after: 47 x 47
+// 1261 and 796 us (memory floor 400), 32 x 32 482 and 421, 16 x 16 256 and 231,
+// 4 x 4 181 and 172; 64 x 64 over 10^6 203 and 147.
 #include "gram_tc.cuh"
 #include "tc.cuh"
 
@@ -45,11 +58,16 @@ namespace {
 
 constexpr int TC_ROLES = 128;  // warps 0-3: producer, MMA issuer, two idle
 constexpr int TC_FLUSH = 4;    // stages per accumulation window (see the precision note)
-constexpr int TC_MAX_SLOTS = 4;
+constexpr int TC_MAX_SLOTS = 6;  // raw tiles in flight
+// Two groups of workers take the stages in turn, each with its own split buffer: a group then waits only
+// for products of its own previous stage, so its parity waits cannot fall a phase behind.
+constexpr int TC_GROUPS = 2;
+constexpr int TC_WORKERS = 256;  // 384 are slower: 929 us for 819, 47 x 47 over 192^3 points
+constexpr int TC_THREADS = TC_ROLES + TC_WORKERS, TC_GROUP_THREADS = TC_WORKERS / TC_GROUPS;
 
 struct GramTcPlan {
-  int a, b, a_pad, b_pad, s, N, slots, tmem_cols;
-  size_t slot_bytes, a_bytes, b_bytes, w_bytes, smem;
+  int a, b, a_pad, a_rows, b_pad, s, N, slots, tmem_cols;
+  size_t slot_bytes, split_bytes, smem;
 };
 
 __host__ __device__ inline int pad_rows(int r) { return r <= 8 ? 8 : r <= 16 ? 16 : r <= 32 ? 32 : 64; }
@@ -59,20 +77,17 @@ bool plan_gram_tc(int a, int b, GramTcPlan* p) {
   p->a = a;
   p->b = b;
   p->a_pad = pad_rows(a);
-  p->b_pad = pad_rows(b);
-  p->s = std::min(128 / p->a_pad, 128 / p->b_pad);  // N <= 128: two accumulator pairs fit 512 columns
+  p->s = std::min(128 / p->a_pad, 128 / pad_rows(b));  // N <= 128: two accumulator pairs fit 512 columns
+  p->a_rows = (a + 7) & ~7;  // rows copied per chunk (whole swizzle atoms); the rest of a_pad stays zero
+  p->b_pad = (b + 7) & ~7;
   p->N = p->s * p->b_pad;
   if (p->N % 16 != 0 || p->N > 128) return false;
-  p->a_bytes = 128 * 128;  // 128 rows x 32 FP32 points
-  p->b_bytes = (size_t)p->N * 128;
-  p->w_bytes = (size_t)32 * p->s * 8;
-  size_t slot = 2 * p->a_bytes + 2 * p->b_bytes + p->w_bytes;
-  slot = (slot + 1023) & ~(size_t)1023;
-  p->slot_bytes = slot;
-  const size_t budget = 220 * 1024;
-  p->slots = (int)std::min<size_t>(TC_MAX_SLOTS, budget / slot);
+  p->slot_bytes = (size_t)p->s * (p->a_rows + p->b_pad) * 128;  // whole 1024-byte swizzle atoms
+  p->split_bytes = 2 * 128 * 128 + 2 * (size_t)p->N * 128;  // A hi, A lo, B hi, B lo; rows of 32 points
+  const size_t budget = 225 * 1024;
+  p->slots = (int)std::min<size_t>(TC_MAX_SLOTS, (budget - TC_GROUPS * p->split_bytes) / p->slot_bytes);
   if (p->slots < 2) return false;
-  p->smem = p->slots * slot + 1024;  // + alignment slack
+  p->smem = p->slots * p->slot_bytes + TC_GROUPS * p->split_bytes + 1024;  // + alignment slack
   int cols = 32;
   while (cols < 4 * p->N) cols <<= 1;
   p->tmem_cols = cols;
@@ -81,54 +96,58 @@ bool plan_gram_tc(int a, int b, GramTcPlan* p) {
 
 struct GramTcArgs {
   long long n;
-  int a, b, a_pad, b_pad, s, N, slots;
-  unsigned slot_bytes, a_bytes, b_bytes;
-  int has_w;
+  int a, b, a_pad, a_rows, b_pad, s, N, slots;
+  unsigned slot_bytes, split_bytes;
+  const double* w;
   long long stages;
   double* part;
   unsigned* err;
 };
 
-template <int NW, int BMAX>
-__global__ void __launch_bounds__(TC_ROLES + NW, 1)
+template <int BMAX>
+__global__ void __launch_bounds__(TC_THREADS, 1)
     gram_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                   const __grid_constant__ CUtensorMap mapW, const GramTcArgs g, uint32_t tmem_cols) {
-  constexpr int TC_THREADS = TC_ROLES + NW;
+                   const GramTcArgs g, uint32_t tmem_cols) {
+  constexpr int NG = TC_GROUP_THREADS;
   extern __shared__ unsigned char tc_smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[TC_MAX_SLOTS], ready_bar[TC_MAX_SLOTS], empty_bar[TC_MAX_SLOTS];
+  __shared__ __align__(8) uint64_t full_bar[TC_MAX_SLOTS], free_bar[TC_MAX_SLOTS];
+  __shared__ __align__(8) uint64_t ready_bar[TC_GROUPS], empty_bar[TC_GROUPS];
   __shared__ __align__(8) uint64_t accf_bar[2], acce_bar[2], done_bar;
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_flag;
   unsigned char* base =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int LS = TC_GROUPS;
   const int S = g.slots;
   const long long G = gridDim.x;
   const long long J = g.stages > blockIdx.x ? (g.stages - blockIdx.x + G - 1) / G : 0;  // stages of this CTA
 
-  auto slotA = [&](int q) { return base + (size_t)q * g.slot_bytes; };
-  auto slotAlo = [&](int q) { return slotA(q) + g.a_bytes; };
-  auto slotB = [&](int q) { return slotA(q) + 2 * g.a_bytes; };
-  auto slotBlo = [&](int q) { return slotB(q) + g.b_bytes; };
-  auto slotW = [&](int q) { return reinterpret_cast<double*>(slotB(q) + 2 * g.b_bytes); };
+  // raw tile of ring slot q: A chunks, B chunks, w; split buffer: A hi, A lo, B hi, B lo
+  auto slotA = [&](int q) { return base + (size_t)LS * g.split_bytes + (size_t)q * g.slot_bytes; };
+  auto slotB = [&](int q) { return slotA(q) + (size_t)g.s * g.a_rows * 128; };
+  auto splitA = [&](int u) { return base + (size_t)u * g.split_bytes; };
+  auto splitB = [&](int u) { return splitA(u) + 2 * 128 * 128; };
 
   if (tid == 0) {
     for (int q = 0; q < S; ++q) {
       mbar_init(&full_bar[q], 1);
-      mbar_init(&ready_bar[q], NW);
-      mbar_init(&empty_bar[q], 1);
+      mbar_init(&free_bar[q], NG / 32);
+    }
+    for (int u = 0; u < LS; ++u) {
+      mbar_init(&ready_bar[u], NG / 32);
+      mbar_init(&empty_bar[u], 1);
     }
     for (int k = 0; k < 2; ++k) {
       mbar_init(&accf_bar[k], 1);
-      mbar_init(&acce_bar[k], 128);  // the four epilogue warps
+      mbar_init(&acce_bar[k], 8);  // the epilogue warps
     }
     mbar_init(&done_bar, 1);
     abort_flag = 0;
     mbar_fence_init();
   }
-  // zero every slot once: A rows past s * a_pad are never written by the
-  // copies and must read as zero; w stays finite where no copy lands
-  for (size_t e = tid; e < (size_t)S * g.slot_bytes / 16; e += TC_THREADS)
+  // zero the split buffers once: rows past the operands' own are never written and must read as zero
+  for (size_t e = tid; e < (size_t)LS * g.split_bytes / 16; e += TC_THREADS)
     reinterpret_cast<uint4*>(base)[e] = make_uint4(0u, 0u, 0u, 0u);
   if (warp == 1) tmem_alloc(&tmem_holder, tmem_cols);
   fence_proxy_async();  // the zero fill is visible to the tensor core and to later copies
@@ -136,23 +155,21 @@ __global__ void __launch_bounds__(TC_ROLES + NW, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_holder;
-  const unsigned tx_bytes = (unsigned)(g.s * (g.a_pad + g.b_pad) * 128 + (g.has_w ? 32 * g.s * 8 : 0));
+  const unsigned tx_bytes = (unsigned)(g.s * (g.a_rows + g.b_pad) * 128);
 
   if (warp == 0 && lane == 0) {
     // ------------------------------------------------ producer
     long long issued = 0;
     for (long long j = 0; j < J; ++j) {
       const int q = (int)(j % S);
-      if (j >= S && !mbar_wait_or_abort(&empty_bar[q], (unsigned)((j / S - 1) & 1), g.err, &abort_flag)) break;
+      if (j >= S && !mbar_wait_or_abort(&free_bar[q], (unsigned)((j / S - 1) & 1), g.err, &abort_flag)) break;
       const long long t = blockIdx.x + j * G;
       const int p0 = (int)(t * 32 * g.s);
       mbar_arrive_expect_tx(&full_bar[q], tx_bytes);
       for (int c = 0; c < g.s; ++c) {
-        tma_load_2d(slotA(q) + (size_t)c * g.a_pad * 128, &mapA, p0 + 32 * c, 0, &full_bar[q]);
+        tma_load_2d(slotA(q) + (size_t)c * g.a_rows * 128, &mapA, p0 + 32 * c, 0, &full_bar[q]);
         tma_load_2d(slotB(q) + (size_t)c * g.b_pad * 128, &mapB, p0 + 32 * c, 0, &full_bar[q]);
       }
-      if (g.has_w)
-        for (int o = 0; o < 32 * g.s; o += 256) tma_load_1d(slotW(q) + o, &mapW, p0 + o, &full_bar[q]);
       issued = j + 1;
     }
     // copies still in flight (after an abort) land before the CTA leaves
@@ -160,28 +177,28 @@ __global__ void __launch_bounds__(TC_ROLES + NW, 1)
       mbar_wait(&full_bar[j % S], (unsigned)((j / S) & 1), g.err);
   } else if (warp == 1 && lane == 0) {
     // ------------------------------------------------ MMA issuer
-    const uint32_t idesc = umma_idesc_tf32(128, g.N);
+    const uint32_t idesc = umma_idesc_tf32(128, g.N), idesc2 = umma_idesc_tf32(128, 2 * g.N);
     for (long long j = 0; j < J; ++j) {
-      const int q = (int)(j % S);
+      const int u = (int)(j % LS);
       const long long win = j / TC_FLUSH;
       const int buf = (int)(win & 1);
       if (j % TC_FLUSH == 0 && win >= 2) {
         if (!mbar_wait_or_abort(&acce_bar[buf], (unsigned)((win / 2 - 1) & 1), g.err, &abort_flag)) break;
       }
-      if (!mbar_wait_or_abort(&ready_bar[q], (unsigned)((j / S) & 1), g.err, &abort_flag)) break;
+      if (!mbar_wait_or_abort(&ready_bar[u], (unsigned)((j / LS) & 1), g.err, &abort_flag)) break;
       tc_fence_after();
       const uint32_t d0 = tmem + (uint32_t)(2 * buf * g.N), d1 = d0 + (uint32_t)g.N;  // hi*hi, cross terms
-      const uint32_t aH = smem_u32(slotA(q)), aL = smem_u32(slotAlo(q));
-      const uint32_t bH = smem_u32(slotB(q)), bL = smem_u32(slotBlo(q));
+      const uint32_t aH = smem_u32(splitA(u)), aL = aH + 128 * 128;
+      const uint32_t bH = smem_u32(splitB(u));
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
         const uint32_t off = kk * 32;  // 8 TF32 values along K
         const uint32_t first = (j % TC_FLUSH == 0 && kk == 0) ? 0u : 1u;
-        umma_tf32(d0, umma_desc_sw128(aH + off), umma_desc_sw128(bH + off), idesc, first);
-        umma_tf32(d1, umma_desc_sw128(aH + off), umma_desc_sw128(bL + off), idesc, first);
+        // [hi*hi | hi*lo] in one product of twice the width: B's lo tile follows its hi tile
+        umma_tf32(d0, umma_desc_sw128(aH + off), umma_desc_sw128(bH + off), idesc2, first);
         umma_tf32(d1, umma_desc_sw128(aL + off), umma_desc_sw128(bH + off), idesc, 1u);
       }
-      umma_commit(&empty_bar[q]);
+      umma_commit(&empty_bar[u]);
       if (j % TC_FLUSH == TC_FLUSH - 1 || j == J - 1) umma_commit(&accf_bar[buf]);
     }
     // every MMA issued has completed before TMEM is released
@@ -189,8 +206,12 @@ __global__ void __launch_bounds__(TC_ROLES + NW, 1)
     mbar_wait(&done_bar, 0u, g.err);
   } else if (warp >= 4) {
     // ------------------------------------------------ split pass + epilogue
-    const int wt = tid - TC_ROLES;         // 0 .. NW-1
-    const bool epi = warp < 8;             // warps 4-7: one per TMEM lane quarter
+    const int wt = tid - TC_ROLES;         // 0 .. TC_WORKERS - 1
+    // warps 4-11: two per TMEM lane quarter, each reads half of a block's columns
+    const bool epi = warp < 12;
+    const int hg = (g.b_pad / 8 + 1) / 2;                       // column groups of 8 of the first half
+    const int jb = warp < 8 ? 0 : 8 * hg;                       // first column of this warp
+    const int jn = warp < 8 ? 8 * hg : g.b_pad - 8 * hg;        // and their number, at most BMAX
     const int m = (warp & 3) * 32 + lane;  // TMEM lane = accumulator row of this thread
     const int my_c = m / g.a_pad, my_i = m % g.a_pad;
     const bool owns_row = epi && my_c < g.s && my_i < g.a;
@@ -202,12 +223,33 @@ __global__ void __launch_bounds__(TC_ROLES + NW, 1)
       cmp[j] = (t - acc[j]) - y;
       acc[j] = t;
     };
-    const int a_chunks = g.s * g.a_pad * 8;  // 16-byte chunks of live A rows
-    // B: thread -> one column group (stack chunk c, logical 16-byte chunk jl: 4 points)
-    // and every (NW / G)-th row of it, so each weight is converted once per thread
+    // Worker group grp splits stages grp, grp + TC_GROUPS, ...  A thread of it takes one column group
+    // (stack chunk bc, logical 16-byte chunk bjl: 4 points) and every rstep-th row of it, so each
+    // weight is converted once per thread
+    const int grp = wt / NG, gt = wt % NG;
     const int G = 8 * g.s;
-    const int grp = wt % G, rstep = NW >= G ? NW / G : 1, r0 = NW >= G ? wt / G : 0;
-    const int bc = grp >> 3, bjl = grp & 7;
+    const int rstep = NG / G, r0 = gt / G;  // powers of two: G <= 128 = NG, rstep <= 8
+    const int bc = (gt % G) >> 3, bjl = gt & 7;
+    // weights of the thread's four points of a stage; zero past the grid, like the copied rows.  Read one
+    // stage ahead, straight from memory (in the ring they would cost it a slot), and converted when used
+    struct W4 {
+      double2 lo, hi;
+    };
+    auto weights = [&](long long j) {
+      const long long p = ((blockIdx.x + j * gridDim.x) * g.s + bc) * 32 + bjl * 4;
+      W4 v = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+      if (g.w && j < J) {
+        if (p + 4 <= g.n) {
+          v.lo = __ldg(reinterpret_cast<const double2*>(g.w + p));
+          v.hi = __ldg(reinterpret_cast<const double2*>(g.w + p) + 1);
+        } else {
+          if (p < g.n) v.lo.x = g.w[p];
+          if (p + 1 < g.n) v.lo.y = g.w[p + 1];
+          if (p + 2 < g.n) v.hi.x = g.w[p + 2];
+        }
+      }
+      return v;
+    };
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     // epilogue of window `win`: TMEM diagonal blocks -> FP64 registers
     auto flush = [&](long long win) -> bool {
@@ -224,9 +266,9 @@ __global__ void __launch_bounds__(TC_ROLES + NW, 1)
         if (c >= g.s) break;  // warp-uniform
 #pragma unroll
         for (int j0 = 0; j0 < BMAX; j0 += 8) {  // compile-time indices keep acc in registers
-          if (j0 < g.b_pad) {
+          if (j0 < jn) {
             float v0[8], v1[8];
-            const uint32_t col = lane_base + (uint32_t)(2 * buf * g.N + c * g.b_pad + j0);
+            const uint32_t col = lane_base + (uint32_t)(2 * buf * g.N + c * g.b_pad + jb + j0);
             tmem_ld8(tmem + col, v0);
             tmem_ld8(tmem + col + (uint32_t)g.N, v1);
             tmem_ld_wait();
@@ -241,7 +283,8 @@ __global__ void __launch_bounds__(TC_ROLES + NW, 1)
         }
       }
       tc_fence_before();
-      mbar_arrive(&acce_bar[buf]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acce_bar[buf]);
       return true;
     };
     // hi = x rounded to the nearest TF32 value (low 13 mantissa bits cleared), lo = x - hi
@@ -256,63 +299,69 @@ __global__ void __launch_bounds__(TC_ROLES + NW, 1)
       l.w = x.w - h.w;
     };
     bool ok = true;
-    for (long long j = 0; j < J && ok; ++j) {
-      const int q = (int)(j % S);
+    long long fw = 0;  // windows read out so far
+    W4 wnext = weights(grp);
+    for (long long j = grp; j < J && ok; j += TC_GROUPS) {
+      const int q = (int)(j % S), u = (int)(j % LS);
       // warp-uniform: every lane of a worker warp leaves the loop in the same stage
-      if (!__all_sync(0xffffffffu, mbar_wait_or_abort(&full_bar[q], (unsigned)((j / S) & 1), g.err, &abort_flag))) {
+      bool go = j < LS || mbar_wait_or_abort(&empty_bar[u], (unsigned)((j / LS - 1) & 1), g.err, &abort_flag);
+      go = go && mbar_wait_or_abort(&full_bar[q], (unsigned)((j / S) & 1), g.err, &abort_flag);
+      if (!__all_sync(0xffffffffu, go)) {
         ok = false;
         break;
       }
-      float4* A4 = reinterpret_cast<float4*>(slotA(q));
-      float4* AL4 = reinterpret_cast<float4*>(slotAlo(q));
+      const float4 wv = g.w ? make_float4((float)wnext.lo.x, (float)wnext.lo.y, (float)wnext.hi.x, (float)wnext.hi.y)
+                            : make_float4(1.f, 1.f, 1.f, 1.f);
+      wnext = weights(j + TC_GROUPS);
+      const float4* A4 = reinterpret_cast<const float4*>(slotA(q)) + bc * g.a_rows * 8;
+      const float4* B4 = reinterpret_cast<const float4*>(slotB(q)) + bc * g.b_pad * 8;
+      float4* A2 = reinterpret_cast<float4*>(splitA(u)) + bc * g.a_pad * 8;
+      float4* B2 = reinterpret_cast<float4*>(splitB(u)) + bc * g.b_pad * 8;
 #pragma unroll 4
-      for (int e = wt; e < a_chunks; e += NW) {
+      for (int r = r0; r < g.a_rows; r += rstep) {
+        const int e = r * 8 + (bjl ^ (r & 7));  // physical 16-byte chunk (128-byte swizzle)
         float4 h, l;
         split4(A4[e], h, l);
-        A4[e] = h;
-        AL4[e] = l;
+        A2[e] = h;
+        A2[128 * 8 + e] = l;
       }
-      float4* B4 = reinterpret_cast<float4*>(slotB(q));
-      float4* BL4 = reinterpret_cast<float4*>(slotBlo(q));
-      if (wt < G * rstep) {
-        float4 wv = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (g.has_w) {
-          const double* wq = slotW(q) + bc * 32 + bjl * 4;
-          wv = make_float4((float)wq[0], (float)wq[1], (float)wq[2], (float)wq[3]);
-        }
 #pragma unroll 4
-        for (int r = r0; r < g.b_pad; r += rstep) {
-          const int ra = bc * g.b_pad + r;
-          const int e = ra * 8 + (bjl ^ (ra & 7));  // physical 16-byte chunk (128-byte swizzle)
-          float4 x = B4[e];
-          x.x *= wv.x;
-          x.y *= wv.y;
-          x.z *= wv.z;
-          x.w *= wv.w;
-          float4 h, l;
-          split4(x, h, l);
-          B4[e] = h;
-          BL4[e] = l;
-        }
+      for (int r = r0; r < g.b_pad; r += rstep) {
+        const int e = r * 8 + (bjl ^ (r & 7));
+        float4 x = B4[e];
+        x.x *= wv.x;
+        x.y *= wv.y;
+        x.z *= wv.z;
+        x.w *= wv.w;
+        float4 h, l;
+        split4(x, h, l);
+        B2[e] = h;
+        B2[g.N * 8 + e] = l;
       }
       fence_proxy_async();  // generic-proxy writes -> visible to the tensor core
-      mbar_arrive(&ready_bar[q]);
-      // read out the previous window once this window's first stage is handed over
-      if (epi && j % TC_FLUSH == 0 && j > 0) ok = flush(j / TC_FLUSH - 1);
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&free_bar[q]);
+        mbar_arrive(&ready_bar[u]);
+      }
+      // read out the finished windows once this group's first stage of the next one is handed over
+      if (epi)
+        for (; ok && fw < j / TC_FLUSH; ++fw) ok = flush(fw);
     }
-    if (epi && ok && J > 0) ok = flush((J - 1) / TC_FLUSH);
+    if (epi)
+      for (; ok && J > 0 && fw <= (J - 1) / TC_FLUSH; ++fw) ok = flush(fw);
     // cross-chunk sum in shared memory (reuses the slots; every MMA has completed)
-    named_bar_sync(1, NW);
+    named_bar_sync(1, TC_WORKERS);
     double* red = reinterpret_cast<double*>(base);
     if (owns_row) {
       double* row = red + ((size_t)my_c * g.a + my_i) * g.b;
 #pragma unroll
       for (int x = 0; x < BMAX; ++x)
-        if (x < g.b) row[x] = (double)acc[x] - (double)cmp[x];
+        if (x < jn && jb + x < g.b) row[jb + x] = (double)acc[x] - (double)cmp[x];
     }
-    named_bar_sync(1, NW);
+    named_bar_sync(1, TC_WORKERS);
     double* pb = g.part + (long long)blockIdx.x * g.a * g.b;
-    for (int e = wt; e < g.a * g.b; e += NW) {
+    for (int e = wt; e < g.a * g.b; e += TC_WORKERS) {
       double v = 0.0;
       for (int c = 0; c < g.s; ++c) v += red[(size_t)c * g.a * g.b + e];
       pb[e] = abort_flag ? 0.0 : v;
@@ -337,11 +386,11 @@ int gram_tc_launch(long long n, int a, int b, const float* A, long long sa, cons
   if (!al16(A) || !al16(B) || (w && !al16(w)) || (sa * 4) % 16 != 0 || (sb * 4) % 16 != 0) return -1;
   if (n < 32 || n >= (1LL << 31) - 4096) return -1;
   if (!err) return IGD_ERR_CUDA;
-  CUtensorMap mA, mB, mW;
+  CUtensorMap mA, mB;
   {
     const unsigned long long dims[2] = {(unsigned long long)n, (unsigned long long)a};
     const unsigned long long strides[1] = {(unsigned long long)sa * 4};
-    const unsigned box[2] = {32, (unsigned)p.a_pad};
+    const unsigned box[2] = {32, (unsigned)p.a_rows};
     if (!encode_tensor_map_ex(&mA, false, 2, A, dims, strides, box, true)) return -1;
   }
   {
@@ -350,38 +399,27 @@ int gram_tc_launch(long long n, int a, int b, const float* A, long long sa, cons
     const unsigned box[2] = {32, (unsigned)p.b_pad};
     if (!encode_tensor_map_ex(&mB, false, 2, B, dims, strides, box, true)) return -1;
   }
-  if (w) {
-    const unsigned long long dims[1] = {(unsigned long long)n};
-    const unsigned box[1] = {(unsigned)std::min(256, 32 * p.s)};
-    if (!encode_tensor_map_ex(&mW, true, 1, w, dims, nullptr, box, false)) return -1;
-  } else {
-    mW = mA;  // unused
-  }
   const int sms = device_sm_count();
-  // up to 32 output columns: 8 worker warps (32 FP64 sums per epilogue thread);
-  // 64 columns: 4 worker warps (64 sums, register budget of 256 threads)
-  const bool wide = p.b_pad > 32;
-  auto kern = wide ? gram_tc_kernel<128, 64> : gram_tc_kernel<256, 32>;
-  const int threads = wide ? TC_ROLES + 128 : TC_ROLES + 256;
+  auto kern = p.b_pad > 32 ? gram_tc_kernel<32> : gram_tc_kernel<16>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), p.smem) != IGD_OK) return IGD_ERR_CUDA;
   GramTcArgs g;
   g.n = n;
   g.a = a;
   g.b = b;
   g.a_pad = p.a_pad;
+  g.a_rows = p.a_rows;
   g.b_pad = p.b_pad;
   g.s = p.s;
   g.N = p.N;
   g.slots = p.slots;
   g.slot_bytes = (unsigned)p.slot_bytes;
-  g.a_bytes = (unsigned)p.a_bytes;
-  g.b_bytes = (unsigned)p.b_bytes;
-  g.has_w = w ? 1 : 0;
+  g.split_bytes = (unsigned)p.split_bytes;
+  g.w = w;
   g.stages = (n + 32LL * p.s - 1) / (32LL * p.s);
   g.part = part;
   g.err = err;
   const int grid = (int)std::max<long long>(1, std::min<long long>({(long long)sms, g.stages, (long long)max_blocks}));
-  kern<<<grid, threads, p.smem, st>>>(mA, mB, mW, g, (uint32_t)p.tmem_cols);
+  kern<<<grid, TC_THREADS, p.smem, st>>>(mA, mB, g, (uint32_t)p.tmem_cols);
   return grid;
 }
 
