@@ -655,18 +655,23 @@ struct LinPlan {
   long long ctas;
 };
 
-// Row tiles and CTAs: the choice whose estimated time is lowest.  A tile's rows share their two
-// halo rows, a share's planes two extra planes and the first loads; both are cheapest when long,
-// while the shares have to fill the SMs.  Costs in SM clocks: `full` per own point (all NB
-// orbitals), `halo` per halo point, `edge` per own point of an extra plane; a march step adds
-// `step` clocks of load, barrier and FP64-chain latency, and a CTA alone on its SM runs `lone`
-// times longer.  Fitted to measured times: FP64 on 67x67x81, 20 orbitals, 6 / 7 / 9 / 12 tiles
-// with two CTAs per SM 307 / 320 / 350 / 347 us (one per SM 346 / 360 / 385), one orbital 7 to 30
-// tiles 32-40 us; FP32 (one CTA per SM), 20 orbitals, 7 / 8 / 9 / 12 tiles 38 / 38 / 40 / 45 us.
+// Row tiles and CTAs: the choice whose estimated time is lowest.  A tile's rows share their halo
+// rows, a share's planes two extra planes and the first loads; both are cheapest when long, while
+// the shares have to fill the SMs.  What decides on small grids is the largest share: with as many
+// CTAs per unit as divide the grid, no share crosses a unit (which would march the extra planes and
+// load the first ones twice).  Costs in SM clocks: `full` per own point (all NB orbitals), `halo` per
+// halo point (its loads included), `edge` per own point of an extra plane; a march step and, `start`
+// times, a segment's first loads add `step` clocks of latency, and a CTA alone on its SM runs `lone`
+// times longer.  Fitted to 400 timed plans of 24 FP64 and 20 FP32 cases (grids of 17 thousand to 1.3
+// million points, 1 to 20 orbitals), whose picks are then within 4 % (FP64) and 6 % (FP32) of the
+// fastest but for 15 % on 25x27x29.  FP64, production closure, with shares cut regardless of the units
+// (two CTAs per SM) / as here: 67x67x81 36.9 / 30.5 us, 57x73x61 30.7 / 21.7, 96x96x96 68.0 / 50.5,
+// 48x80x150 69.7 / 40.5, eight orbitals on 45x51x47 61.5 / 49.1, 20 on 25x27x29 50.7 / 31.5, 20 on
+// 67x67x81 317 either way; FP32, one orbital on 57x73x61 10.4 / 9.4, eight on 45x51x47 14.0 / 11.8.
 struct LinCost {
   int oycap, maxres, values;  // tallest tile, CTAs per SM, shared values per cell
   size_t value_bytes;
-  double full, halo, edge, step, lone;
+  double full, halo, edge, step, start, lone;
 };
 
 template <typename CELLS>
@@ -678,21 +683,35 @@ LinPlan lin_search(int nx, int ny, int nz, int groups, CELLS cells, const LinCos
     const int oy = (ny + tiles - 1) / tiles;  // tallest tile
     const int res = (int)std::min<size_t>(c.maxres, 227 * 1024 / (cells(oy, nz) * c.values * c.value_bytes + 1024));
     if (res < 1) continue;
-    const long long total = (long long)tiles * groups * nx, units = (long long)tiles * groups;
+    const long long units = (long long)tiles * groups, total = units * nx;
     if (total > 0x3fffffff) break;
-    const double pl = (c.full * ny / tiles + 2 * c.halo) * nz, ed = c.edge * ny / tiles * nz;
-    for (int r = res; r >= 1; --r) {
-      for (int least = 1; least <= 4; least *= 2) {  // planes a share has at least
-        const long long ctas = std::max(1LL, std::min((long long)sms * r, total / least));
-        const double share = (double)total / ctas, segs = 1.0 + (double)units / ctas;
-        const long long per_sm = (ctas + sms - 1) / sms;
-        const double t =
-            (per_sm == 1 ? c.lone : (double)per_sm) * (share * pl + segs * 2 * ed) + (share + 4 * segs) * c.step;
-        if (best.tiles == 0 || t < tbest) {
-          tbest = t;
-          best = LinPlan{oy, tiles, ctas};
-        }
+    const double pl = (c.full * ny / tiles + 2 * c.halo) * nz, ed = c.edge * oy * nz;
+    auto consider = [&](long long ctas) {
+      if (ctas < 1 || ctas > total) return;
+      long long share = (total + ctas - 1) / ctas;  // planes of the largest share
+      double segs = 2.0 + (double)(share / nx);
+      if (ctas % units == 0) {
+        segs = 1.0;
+        share = (nx + ctas / units - 1) / (ctas / units);
+      } else if (units % ctas == 0) {
+        segs = (double)(units / ctas);
       }
+      const long long per_sm = (ctas + sms - 1) / sms;
+      const double t = (per_sm == 1 ? c.lone : (double)per_sm) * (share * pl + segs * 2 * ed) +
+                       (share + c.start * segs) * c.step;
+      if (best.tiles == 0 || t < tbest) {
+        tbest = t;
+        best = LinPlan{oy, tiles, ctas};
+      }
+    };
+    for (int r = res; r >= 1; --r) {
+      const long long cap = (long long)sms * r;
+      consider(std::min(cap, total));
+      for (int least = 2; least <= 4; ++least) consider(std::min(cap, (total + least - 1) / least));
+      if (units <= cap)
+        consider(cap / units * units);
+      else
+        consider(units / ((units + cap - 1) / cap));
     }
   }
   return best;
@@ -744,8 +763,8 @@ int lin64_launch(const double* coeffs, const double* veff, const double* psi, do
   --kexp;
   if (kexp < -32 || kexp > 32) return -1;
   const LinPlan p = lin_plan(nx, ny, nz, nb, lin64_cells,
-                             LinCost{std::min(ny, L64_NT * L64_PPT / nz), L64_MINB, 1, sizeof(double), 10.5, 3.0, 3.0,
-                                     3000.0, 1.25});
+                             LinCost{std::min(ny, L64_NT * L64_PPT / nz), L64_MINB, 1, sizeof(double), 10.5, 28.6, 13.5,
+                                     1600.0, 3.3, 1.16});
   if (p.tiles == 0) return -1;
   const size_t smem = lin64_cells(p.oymax, nz) * sizeof(double);
   auto kern = hpsi_lin64_kernel<PROD, KRY, HASV>;
@@ -770,7 +789,8 @@ int lin32_launch(const float* coeffs, const float* veff, const float* psi, float
   const int groups = (nb + NB - 1) / NB;
   const double pt = 0.6 + 0.7 * NB;
   const LinPlan p = lin_plan(nx, ny, nz, groups, lin32_cells<NB>,
-                             LinCost{std::min(ny, L32_NT * PPT / nz - 2), 1, NB, sizeof(float), pt, pt, pt, 600.0, 1.0});
+                             LinCost{std::min(ny, L32_NT * PPT / nz - 2), 1, NB, sizeof(float), pt, 1.8 * pt, 0.85 * pt,
+                                     1250.0, 4.5, 1.0});
   if (p.tiles == 0) return -1;
   const size_t smem = lin32_cells<NB>(p.oymax, nz) * sizeof(float) * NB;
   auto kern = hpsi_lin32_kernel<NB, PPT, PROD, KRY>;
