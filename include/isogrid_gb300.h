@@ -206,6 +206,10 @@ int igd_lsda(int dtype, int math, int functional, long long n, const void* rho_u
  * (_build_density_from_occupied_orbitals, scf/driver.py:663-676). */
 int igd_density(int dtype, long long n, int nb, long long stride, const void* psi, const double* occupations,
                 const double* w, double* rho, double* integral, int accumulate, void* stream);
+/* The same with at most IGD_DENSITY_VALUES occupations, read from host memory before the call returns. */
+#define IGD_DENSITY_VALUES 64
+int igd_density_values(int dtype, long long n, int nb, long long stride, const void* psi, const double* occupations,
+                       const double* w, double* rho, double* integral, int accumulate, void* stream);
 /* rho *= target / *integral on the device (_renormalize_density, scf/driver.py:679-690). */
 int igd_density_renormalize(long long n, double* rho, const double* integral, double target, int* flags,
                             void* stream);

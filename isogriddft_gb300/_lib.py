@@ -12,6 +12,7 @@ import os
 LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libisogrid_gb300.so")
 
 IGD_OK, IGD_ERR_ARG, IGD_ERR_DTYPE, IGD_ERR_CUDA, IGD_ERR_BREAKDOWN, IGD_ERR_NOT_CONVERGED, IGD_ERR_NONFINITE, IGD_ERR_TOO_LARGE = range(8)
+IGD_DENSITY_VALUES = 64  # occupations that igd_density_values takes
 IGD_F32, IGD_F64 = 0, 1
 IGD_CLOSURE_TRIAL_FIX, IGD_CLOSURE_PRODUCTION = 0, 1
 IGD_GRID_MONITOR, IGD_GRID_LEGACY = 0, 1
@@ -45,6 +46,7 @@ SIGNATURES: dict[str, list] = {
     "igd_weighted_sum": [_c_int, _c_ll, _vp, _vp, _vp, _vp, _vp],
     "igd_lsda": [_c_int, _c_int, _c_int, _c_ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "igd_density": [_c_int, _c_ll, _c_int, _c_ll, _vp, _vp, _vp, _vp, _vp, _c_int, _vp],
+    "igd_density_values": [_c_int, _c_ll, _c_int, _c_ll, _vp, _vp, _vp, _vp, _vp, _c_int, _vp],
     "igd_density_renormalize": [_c_ll, _vp, _vp, _c_dbl, _vp, _vp],
     "igd_density_residual2": [_c_ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "igd_gram_select": [_c_int],

@@ -320,18 +320,25 @@ __global__ void __launch_bounds__(XB, 3) lsda64_kernel(long long n, const T* __r
   if (fl) atomicOr(flags, fl);
 }
 
-constexpr int DENS_MAXNB = 64;  // occupations held in shared memory
+constexpr int DENS_MAXNB = IGD_DENSITY_VALUES;  // occupations held in shared memory
+
+// Where a density kernel's occupations come from: device memory, or (p null) the launch's own arguments.
+struct Occupations {
+  const double* p;
+  double v[DENS_MAXNB];
+  __device__ __forceinline__ double at(int o) const { return p ? p[o] : v[o]; }
+};
 
 // rho = sum_i occ_i psi_i^2 (FP64 out); *integral += sum rho W.  Up to DENS_MAXNB occupations are
 // converted to the orbital type once per block (SHARED): converted at every point they kept the FP64
 // pipe busy.  16 FP32 orbitals over 127^3 points: 75.9 us, now 32.9 (memory floor 24).
 template <typename T, bool SHARED>
 __global__ void density_kernel(long long n, int nb, long long stride, const T* __restrict__ psi,
-                               const double* __restrict__ occ, const double* __restrict__ w, double* __restrict__ rho,
-                               double* integral, int accumulate) {
+                               const __grid_constant__ Occupations occ, const double* __restrict__ w,
+                               double* __restrict__ rho, double* integral, int accumulate) {
   __shared__ T so[SHARED ? DENS_MAXNB : 1];
   if constexpr (SHARED) {
-    for (int o = threadIdx.x; o < nb; o += blockDim.x) so[o] = T(occ[o]);
+    for (int o = threadIdx.x; o < nb; o += blockDim.x) so[o] = T(occ.at(o));
     __syncthreads();
   }
   double acc = 0.0;
@@ -342,7 +349,7 @@ __global__ void density_kernel(long long n, int nb, long long stride, const T* _
 #pragma unroll 8
     for (int o = 0; o < nb; ++o) {
       const T p = psi[(long long)o * stride + i];
-      t += (SHARED ? so[o] : T(occ[o])) * p * p;
+      t += (SHARED ? so[o] : T(occ.p[o])) * p * p;
     }
     const double r = (accumulate ? rho[i] : 0.0) + (double)t;
     rho[i] = r;
@@ -361,10 +368,10 @@ __global__ void density_kernel(long long n, int nb, long long stride, const T* _
 // FP64 density and integral.  The orbital loop is unrolled by 16 to have enough loads in
 // flight: 16 orbitals over 128^3 points 43.6 us with 4, 40.5 with 8, 36.0 with 16 (memory floor 25).
 __global__ void density_v4_kernel(long long n4, int nb, long long stride, const float* __restrict__ psi,
-                                  const double* __restrict__ occ, const double* __restrict__ w,
+                                  const __grid_constant__ Occupations occ, const double* __restrict__ w,
                                   double* __restrict__ rho, double* integral, int accumulate) {
   __shared__ float so[DENS_MAXNB];
-  for (int o = threadIdx.x; o < nb; o += blockDim.x) so[o] = (float)occ[o];
+  for (int o = threadIdx.x; o < nb; o += blockDim.x) so[o] = (float)occ.at(o);
   __syncthreads();
   double acc = 0.0;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
@@ -488,13 +495,8 @@ extern "C" int igd_lsda(int dtype, int math, int functional, long long n, const 
   return launch_status();
 }
 
-// rho (FP64, n) = [rho +] sum_i occupations[i] psi_i^2 over nb orbitals of `dtype`
-// separated by stride elements; occupations: nb device doubles.  integral (device,
-// may be NULL) = sum rho W (zeroed first).
-extern "C" int igd_density(int dtype, long long n, int nb, long long stride, const void* psi, const double* occupations,
-                           const double* w, double* rho, double* integral, int accumulate, void* stream) {
-  if (n <= 0 || nb < 0 || !rho || (nb > 0 && (!psi || !occupations))) return IGD_ERR_ARG;
-  cudaStream_t st = as_stream(stream);
+static int density_launch(int dtype, long long n, int nb, long long stride, const void* psi, const Occupations& occupations,
+                          const double* w, double* rho, double* integral, int accumulate, cudaStream_t st) {
   if (integral) zero1<<<1, 1, 0, st>>>(integral);
   auto plain = [&](auto zero) {
     using T = decltype(zero);
@@ -514,6 +516,27 @@ extern "C" int igd_density(int dtype, long long n, int nb, long long stride, con
   else
     return IGD_ERR_DTYPE;
   return launch_status();
+}
+
+// rho (FP64, n) = [rho +] sum_i occupations[i] psi_i^2 over nb orbitals of `dtype`
+// separated by stride elements; occupations: nb device doubles.  integral (device,
+// may be NULL) = sum rho W (zeroed first).
+extern "C" int igd_density(int dtype, long long n, int nb, long long stride, const void* psi, const double* occupations,
+                           const double* w, double* rho, double* integral, int accumulate, void* stream) {
+  if (n <= 0 || nb < 0 || !rho || (nb > 0 && (!psi || !occupations))) return IGD_ERR_ARG;
+  Occupations occ{};
+  occ.p = nb ? occupations : nullptr;
+  return density_launch(dtype, n, nb, stride, psi, occ, w, rho, integral, accumulate, as_stream(stream));
+}
+
+// The same with the occupations (at most IGD_DENSITY_VALUES host doubles) in the launch's arguments.
+extern "C" int igd_density_values(int dtype, long long n, int nb, long long stride, const void* psi,
+                                  const double* occupations, const double* w, double* rho, double* integral,
+                                  int accumulate, void* stream) {
+  if (n <= 0 || nb < 0 || nb > DENS_MAXNB || !rho || (nb > 0 && (!psi || !occupations))) return IGD_ERR_ARG;
+  Occupations occ{};
+  for (int o = 0; o < nb; ++o) occ.v[o] = occupations[o];
+  return density_launch(dtype, n, nb, stride, psi, occ, w, rho, integral, accumulate, as_stream(stream));
 }
 
 // rho *= target / *integral on the device (flags |= 4 when the integral is not positive).

@@ -20,14 +20,22 @@ from .ops import validate_orbital_field
 def build_density_device(dg, orbitals: torch.Tensor, occupations, *, out: torch.Tensor | None = None,
                          accumulate: bool = False, integral: torch.Tensor | None = None) -> torch.Tensor:
     nb = 0 if orbitals is None else orbitals.shape[0]
-    occ = torch.as_tensor(np.asarray(occupations, dtype=np.float64), device=dg.device)
-    if len(occ) < nb:
-        nb = len(occ)
-    if out is None:
-        out = torch.zeros(dg.n, dtype=torch.float64, device=dg.device)
+    occ = np.asarray(occupations, dtype=np.float64)
+    nb = min(nb, len(occ))
+    occ = np.ascontiguousarray(occ)
+    if out is None:  # written whole unless it is added to
+        out = (torch.zeros if accumulate else torch.empty)(dg.n, dtype=torch.float64, device=dg.device)
     dt = _lib.IGD_F32 if (orbitals is not None and orbitals.dtype == torch.float32) else _lib.IGD_F64
-    _lib.check(_lib.call("igd_density", dt, dg.n, nb, dg.n, ptr(orbitals) if nb else None, ptr(occ) if nb else None,
-                         ptr(dg.cell_volumes), ptr(out), ptr(integral), int(accumulate), stream_ptr()), "igd_density")
+    st = stream_ptr()
+    if nb <= _lib.IGD_DENSITY_VALUES:
+        # occupations by value with the launch: the copy of a small array costs 19 us
+        status = _lib.call("igd_density_values", dt, dg.n, nb, dg.n, ptr(orbitals) if nb else None, occ.ctypes.data,
+                           ptr(dg.cell_volumes), ptr(out), ptr(integral), int(accumulate), st)
+    else:
+        occ = torch.as_tensor(occ, device=dg.device)
+        status = _lib.call("igd_density", dt, dg.n, nb, dg.n, ptr(orbitals), ptr(occ), ptr(dg.cell_volumes), ptr(out),
+                           ptr(integral), int(accumulate), st)
+    _lib.check(status, "igd_density")
     return out
 
 
@@ -35,10 +43,10 @@ def renormalize_device(dg, rho: torch.Tensor, target: float, integral: torch.Ten
     if target == 0.0:
         rho.zero_()
         return rho
-    flags = torch.zeros(1, dtype=torch.int32, device=dg.device)
+    flags = torch.empty(1, dtype=torch.int32, device=dg.device)  # not read: the integral says the same
     _lib.check(_lib.call("igd_density_renormalize", dg.n, ptr(rho), ptr(integral), float(target), ptr(flags),
                          stream_ptr()), "igd_density_renormalize")
-    if int(flags.item()) & 4:
+    if not (integral if integral.numel() == 1 else integral.reshape(-1)[0]).item() > 0.0:
         raise ValueError("A positive density integral is required for renormalization.")
     return rho
 

@@ -29,6 +29,7 @@ def require_cuda() -> torch.device:
     return torch.device("cuda", torch.cuda.current_device())
 
 
+_RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _HELD = threading.local()  # per thread: the stream fixed by held_stream(), if any
 
 
@@ -38,6 +39,8 @@ def stream_ptr() -> int:
     fixed = getattr(_HELD, "stream", None)
     if fixed is not None:
         return fixed
+    if _RAW_STREAM is not None:  # 0.9 us with the device lookup; the Stream object takes 3.4
+        return _RAW_STREAM(torch.cuda.current_device())
     return torch.cuda.current_stream().cuda_stream
 
 

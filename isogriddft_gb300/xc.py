@@ -56,7 +56,7 @@ def lsda_device(rho_up: torch.Tensor, rho_down: torch.Tensor, *, functional: str
             raise ValueError(f"{name} must be a contiguous CUDA field of {n} points like rho_up; received shape "
                              f"{tuple(t.shape)}, {t.dtype} on {t.device}.")
     out ={k: (torch.empty_like(rho_up) if k in want else None) for k in ("eps", "v_up", "v_down", "edens")}
-    energy = torch.zeros(1, dtype=torch.float64, device=rho_up.device) if w is not None else None
+    energy = torch.empty(1, dtype=torch.float64, device=rho_up.device) if w is not None else None
     flags = torch.zeros(1, dtype=torch.int32, device=rho_up.device)
     _lib.check(_lib.call("igd_lsda", dt, mt, fid, n, ptr(rho_up), ptr(rho_down), ptr(out["eps"]), ptr(out["v_up"]),
                          ptr(out["v_down"]), ptr(out["edens"]), ptr(w), ptr(energy), ptr(flags), stream_ptr()),

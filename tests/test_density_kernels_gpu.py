@@ -1,9 +1,12 @@
 """Density kernels: shared and direct occupations, ragged grids and strides; renormalisation of even and odd grids."""
 
+from types import SimpleNamespace
+
+import numpy as np
 import pytest
 import torch
 
-from isogriddft_gb300 import _lib
+from isogriddft_gb300 import _lib, density
 from isogriddft_gb300.device import ptr, stream_ptr
 
 pytestmark = pytest.mark.gpu
@@ -49,3 +52,30 @@ def test_renormalisation(n):
             kept = rho.clone()
             call()
             assert torch.equal(rho, kept) and int(flags) == 4
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("nb,count", [(0, 0), (3, 3), (5, 2), (2, 5), (64, 64), (65, 65), (70, 64)])
+def test_occupations_by_value_and_from_memory_agree(nb, count, dtype):
+    n = 4099
+    dg = SimpleNamespace(n=n, device=torch.device("cuda", 0),
+                         cell_volumes=torch.rand(n, device="cuda", dtype=torch.float64))
+    psi = torch.randn(nb, n, device="cuda", dtype=dtype) if nb else None
+    occ = np.random.default_rng(nb).random(2 * count)[::2]  # a strided array
+    used = min(nb, count)
+    dev_occ = torch.as_tensor(np.ascontiguousarray(occ), device="cuda")
+    want = torch.zeros(n, device="cuda", dtype=torch.float64)
+    code = _lib.IGD_F32 if dtype == torch.float32 and nb else _lib.IGD_F64
+    _lib.check(_lib.call("igd_density", code, n, used, n, ptr(psi) if used else None, ptr(dev_occ) if used else None,
+                         ptr(dg.cell_volumes), ptr(want), None, 0, stream_ptr()))
+    integral = torch.empty(1, device="cuda", dtype=torch.float64)
+    assert torch.equal(density.build_density_device(dg, psi, occ, integral=integral), want)
+    assert torch.equal(density.build_density_device(dg, psi, list(occ)), want)
+    twice = density.build_density_device(dg, psi, occ, out=want.clone(), accumulate=True)
+    assert torch.equal(twice, want + want)
+    if used:
+        scaled = density.renormalize_device(dg, want.clone(), 2.0, integral)
+        assert torch.equal(scaled, want * (2.0 / integral.item()))
+    else:
+        with pytest.raises(ValueError, match="positive density integral"):
+            density.renormalize_device(dg, want, 2.0, integral)
