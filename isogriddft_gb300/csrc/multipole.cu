@@ -53,70 +53,118 @@ __global__ void nodal_moments_kernel(long long n, const double* __restrict__ rho
   flush<10>(m, out);
 }
 
-__device__ __forceinline__ double tri(const double c[8], double u, double v, double t) {
-  const double um = 1.0 - u, vm = 1.0 - v, tm = 1.0 - t;
-  return um * vm * tm * c[0] + u * vm * tm * c[1] + um * v * tm * c[2] + u * v * tm * c[3] + um * vm * t * c[4] +
-         u * vm * t * c[5] + um * v * t * c[6] + u * v * t * c[7];
-}
+// Basis functions 1, u, v, t, uu, vv, tt, uv, ut, vt and the index of the product of two of them among
+// the 35 distinct monomials of degree 0 to 4, ordered as the 10 basis functions and then degrees 3 and 4.
+struct QuadTable {
+  int at[10][10] = {};
+  int f1[35] = {}, f2[35] = {};  // a pair of basis functions whose product is the monomial
+  constexpr QuadTable() {
+    const int e[10][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {2, 0, 0},
+                          {0, 2, 0}, {0, 0, 2}, {1, 1, 0}, {1, 0, 1}, {0, 1, 1}};
+    int seen[35][3] = {}, n = 0;
+    for (int a = 0; a < 10; ++a)
+      for (int b = 0; b < 10; ++b) {
+        int k = 0;
+        while (k < n && !(seen[k][0] == e[a][0] + e[b][0] && seen[k][1] == e[a][1] + e[b][1] &&
+                          seen[k][2] == e[a][2] + e[b][2]))
+          ++k;
+        if (k == n) {
+          for (int c = 0; c < 3; ++c) seen[n][c] = e[a][c] + e[b][c];
+          f1[n] = a;
+          f2[n] = b;
+          ++n;
+        }
+        at[a][b] = k;
+      }
+  }
+};
 
 // Least-squares quadratic through the 64 nodes around cell (i, j, k); returns
 // coefficients in local coordinates xi = (r - c) / L.  Normal equations with
-// Cholesky in FP64 (the local scaling keeps them well conditioned).
-__device__ bool quad_fit(const double* __restrict__ X, const double* __restrict__ Y, const double* __restrict__ Z,
-                         const double* __restrict__ R, int ny, int nz, int i, int j, int k, double c[3], double L,
-                         double coef[10]) {
-  double G[55];
-  double b[10];
+// Cholesky in FP64 (the local scaling keeps them well conditioned).  The FP64 pipe
+// bounds it: the 55 products of two basis functions are 35 distinct monomials, whose
+// sums are accumulated once each; the coordinates are scaled by 1 / L and the factor's
+// columns by the reciprocals of its diagonal (a division takes a dozen FP64
+// instructions); and everything is unrolled, so that the matrix stays in registers.
+__device__ __forceinline__ bool quad_fit(const double* __restrict__ X, const double* __restrict__ Y,
+                                         const double* __restrict__ Z, const double* __restrict__ R, int ny, int nz,
+                                         int i, int j, int k, const double (&c)[3], double rL, double (&coef)[10]) {
+  constexpr QuadTable tab;
+  double S[35], b[10];
 #pragma unroll
-  for (int a = 0; a < 55; ++a) G[a] = 0.0;
+  for (int a = 0; a < 35; ++a) S[a] = 0.0;
 #pragma unroll
   for (int a = 0; a < 10; ++a) b[a] = 0.0;
   const long long pl = (long long)ny * nz;
+#pragma unroll 1
   for (int di = -1; di <= 2; ++di)
+#pragma unroll 1
     for (int dj = -1; dj <= 2; ++dj)
+#pragma unroll
       for (int dk = -1; dk <= 2; ++dk) {
         const long long g = (long long)(i + di) * pl + (long long)(j + dj) * nz + (k + dk);
-        const double u = (X[g] - c[0]) / L, v = (Y[g] - c[1]) / L, t = (Z[g] - c[2]) / L;
+        const double u = (X[g] - c[0]) * rL, v = (Y[g] - c[1]) * rL, t = (Z[g] - c[2]) * rL;
         const double f[10] = {1.0, u, v, t, u * u, v * v, t * t, u * v, u * t, v * t};
         const double rv = R[g];
-        int idx = 0;
+        b[0] += rv;
 #pragma unroll
-        for (int a = 0; a < 10; ++a) {
+        for (int a = 1; a < 10; ++a) {
           b[a] += f[a] * rv;
-#pragma unroll
-          for (int e = 0; e <= a; ++e) G[idx++] += f[a] * f[e];
+          S[a] += f[a];
         }
+#pragma unroll
+        for (int a = 10; a < 35; ++a) S[a] += f[tab.f1[a]] * f[tab.f2[a]];
       }
-  // Cholesky G = L L^T in place (packed lower), then solve.
-  int ia = 0;
+  S[0] = 64.0;
+  // Cholesky G = L L^T (packed lower, the diagonal as reciprocals), then solve.
+  double G[55], y[10];
+  bool ok = true;
+#pragma unroll
   for (int a = 0; a < 10; ++a) {
-    const int rowa = a * (a + 1) / 2;
+#pragma unroll
     for (int e = 0; e <= a; ++e) {
-      const int rowe = e * (e + 1) / 2;
-      double s = G[rowa + e];
-      for (int q = 0; q < e; ++q) s -= G[rowa + q] * G[rowe + q];
+      double s = S[tab.at[a][e]];
+#pragma unroll
+      for (int q = 0; q < e; ++q) s -= G[a * (a + 1) / 2 + q] * G[e * (e + 1) / 2 + q];
       if (a == e) {
-        if (!(s > 0.0)) return false;
-        G[rowa + a] = sqrt(s);
+        ok = ok && s > 0.0;
+        G[a * (a + 1) / 2 + a] = 1.0 / sqrt(s);
       } else {
-        G[rowa + e] = s / G[rowe + e];
+        G[a * (a + 1) / 2 + e] = s * G[e * (e + 1) / 2 + e];
       }
     }
-    ia += a + 1;
-  }
-  double y[10];
-  for (int a = 0; a < 10; ++a) {
-    const int rowa = a * (a + 1) / 2;
     double s = b[a];
-    for (int q = 0; q < a; ++q) s -= G[rowa + q] * y[q];
-    y[a] = s / G[rowa + a];
+#pragma unroll
+    for (int q = 0; q < a; ++q) s -= G[a * (a + 1) / 2 + q] * y[q];
+    y[a] = s * G[a * (a + 1) / 2 + a];
   }
+#pragma unroll
   for (int a = 9; a >= 0; --a) {
     double s = y[a];
+#pragma unroll
     for (int q = a + 1; q < 10; ++q) s -= G[q * (q + 1) / 2 + a] * coef[q];
-    coef[a] = s / G[a * (a + 1) / 2 + a];
+    coef[a] = s * G[a * (a + 1) / 2 + a];
   }
-  return true;
+  return ok;
+}
+
+// Trilinear values of a cell's corners c (x fastest) at the eight samples 1/4, 3/4 per axis, one axis
+// after the other: 48 operations instead of eight times eight products.
+__device__ __forceinline__ void tri8(const double (&c)[8], double (&o)[8]) {
+  double x[8], y[8];
+  auto lerp = [](double a, double b, double& lo, double& hi) {
+    lo = fma(0.25, b, 0.75 * a);
+    hi = fma(0.75, b, 0.25 * a);
+  };
+#pragma unroll
+  for (int q = 0; q < 4; ++q) lerp(c[2 * q], c[2 * q + 1], x[2 * q], x[2 * q + 1]);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int a = (q >> 1) * 4 + (q & 1);
+    lerp(x[a], x[a + 2], y[a], y[a + 2]);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) lerp(y[q], y[q + 4], o[q], o[q + 4]);
 }
 
 // mode 0: corrected moments (weight rho_quad J dV about center);
@@ -131,20 +179,18 @@ __global__ void cell_quadrature_kernel(int nx, int ny, int nz, const double* __r
   const long long pl = (long long)ny * nz;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ncells; t += gridDim.x * blockDim.x) {
     const int i = cells[3 * t], j = cells[3 * t + 1], k = cells[3 * t + 2];
-    double cx8[8], cy8[8], cz8[8], cj8[8], cr8[8];
-    int q = 0;
-    for (int dk = 0; dk < 2; ++dk)
-      for (int dj = 0; dj < 2; ++dj)
-        for (int di = 0; di < 2; ++di) {
-          const long long g = (long long)(i + di) * pl + (long long)(j + dj) * nz + (k + dk);
-          cx8[q] = X[g];
-          cy8[q] = Y[g];
-          cz8[q] = Z[g];
-          cj8[q] = J[g];
-          cr8[q] = R[g];
-          ++q;
-        }
+    // corner q = (di, dj, dk), di fastest
+    auto corners = [&](const double* __restrict__ F, double (&o)[8]) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        o[q] = F[(long long)(i + (q & 1)) * pl + (long long)(j + ((q >> 1) & 1)) * nz + (k + (q >> 2))];
+    };
+    double cx8[8], cy8[8], cz8[8];
+    corners(X, cx8);
+    corners(Y, cy8);
+    corners(Z, cz8);
     double c[3] = {0, 0, 0};
+#pragma unroll
     for (int a = 0; a < 8; ++a) {
       c[0] += cx8[a];
       c[1] += cy8[a];
@@ -154,18 +200,29 @@ __global__ void cell_quadrature_kernel(int nx, int ny, int nz, const double* __r
     c[1] *= 0.125;
     c[2] *= 0.125;
     const double Ls = fmax(fmax(fabs(cx8[7] - cx8[0]), fabs(cy8[7] - cy8[0])), fabs(cz8[7] - cz8[0])) + 1e-300;
+    const double rL = 1.0 / Ls;
     double coef[10];
-    if (!quad_fit(X, Y, Z, R, ny, nz, i, j, k, c, Ls, coef)) {
+    if (!quad_fit(X, Y, Z, R, ny, nz, i, j, k, c, rL, coef)) {
       atomicOr(fail, 1);
       continue;
     }
-    for (int s = 0; s < 8; ++s) {
-      const double u = ((s >> 2) & 1) ? 0.75 : 0.25;  // sample (ix, iy, iz) with z fastest
-      const double v = ((s >> 1) & 1) ? 0.75 : 0.25;
-      const double w = (s & 1) ? 0.75 : 0.25;
-      const double xs = tri(cx8, u, v, w), ys = tri(cy8, u, v, w), zs = tri(cz8, u, v, w);
-      const double js = tri(cj8, u, v, w), rt = tri(cr8, u, v, w);
-      const double a = (xs - c[0]) / Ls, b = (ys - c[1]) / Ls, d = (zs - c[2]) / Ls;
+    double sx[8], sy[8], sz[8], sj[8], sr[8], corner[8];
+    corners(X, corner);
+    tri8(corner, sx);
+    corners(Y, corner);
+    tri8(corner, sy);
+    corners(Z, corner);
+    tri8(corner, sz);
+    corners(J, corner);
+    tri8(corner, sj);
+    if (mode != 0) {
+      corners(R, corner);
+      tri8(corner, sr);
+    }
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {  // samples in the corners' order
+      const double xs = sx[s], ys = sy[s], zs = sz[s], js = sj[s], rt = mode != 0 ? sr[s] : 0.0;
+      const double a = (xs - c[0]) * rL, b = (ys - c[1]) * rL, d = (zs - c[2]) * rL;
       const double rq = coef[0] + coef[1] * a + coef[2] * b + coef[3] * d + coef[4] * a * a + coef[5] * b * b +
                         coef[6] * d * d + coef[7] * a * b + coef[8] * a * d + coef[9] * b * d;
       if (mode == 0) {
