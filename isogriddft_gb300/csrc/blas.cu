@@ -23,7 +23,8 @@ thread_local int g_gram_last = 0;                   // kernel of this thread's l
 // FP64: the splitting kernel takes about 22 clocks a point for every 16 x 24 outputs (splitting) plus
 // 8 (row exponents), the plain kernels 0.57 a point and output (FP64 pipe).  363609 points, plain /
 // split: 4 x 4 99 / 46 us (launch-bound plain grid), 8 x 8 99 / 48, 12 x 12 187 / 64, 21 x 21
-// 538 / 140, 34 x 34 1141 / 346; 2000003 points: 4 x 4 122 / 173, 8 x 8 376 / 202.  It would pay from
+// 538 / 140, 34 x 34 1141 / 346; 2000003 points: 4 x 4 122 / 173, 8 x 8 376 / 202 (the plain kernel is
+// 8 % faster since its sums over lanes were shortened).  It would pay from
 // about a thousand points on (20001 points, 21 x 21: 72 / 29 us), but its correctly rounded sums
 // differ from the plain ones in the last bit, and on small grids an eigensolve of a closure that is
 // not self-adjoint turns that into 1e-8 of an unconverged orbital; below the size where the FP32
@@ -33,11 +34,39 @@ inline bool gram64_split_pays(long long n, int a, int b) {
 }
 constexpr int GPT = 64;    // points per thread and block column (FP32 partial sums stay short)
 
+// FP64 <-> FP32 conversions on the integer ALUs (a converted value takes 16 clocks of the SM's FP64 pipe
+// per warp); zeros apart, values outside the normal range go through the instruction, in a call.
+__device__ __noinline__ float narrow_slow(double x) { return (float)x; }
+__device__ __noinline__ double widen_slow(float x) { return (double)x; }
+__device__ __forceinline__ float narrow(double x) {  // to nearest, ties to even
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), e = (hi >> 20) & 0x7ffu;
+  if (e - 897u > 253u) return narrow_slow(x);
+  unsigned f = (((hi & 0x7fffffffu) - 0x38000000u) << 3) | (lo >> 29);
+  const unsigned rest = lo & 0x1fffffffu;
+  f += rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u;
+  return __uint_as_float(f | (hi & 0x80000000u));
+}
+__device__ __forceinline__ double narrow(double x, double) { return x; }
+__device__ __forceinline__ float narrow(double x, float) { return narrow(x); }
+__device__ __forceinline__ double widen(double x) { return x; }
+__device__ __forceinline__ double widen(float x) {
+  const unsigned u = __float_as_uint(x), e = (u >> 23) & 0xffu;
+  if ((u << 1) == 0u) return __hiloint2double((int)u, 0);
+  if (e - 1u > 253u) return widen_slow(x);
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+
 // Register-tiled tall-skinny Gram.  Block (x, y): tile y of TR x TR outputs
 // (rows i0.., columns j0..) over the points of column slice x; each thread
 // streams its points straight from global memory (TR + TR + 1 coalesced loads,
 // TR^2 FMAs per point) into TR^2 register accumulators of T, then the block
-// reduces them in FP64 into part[x][a][b].
+// reduces them in FP64 into part[x][a][b].  The FP64 pipe bounded the FP32 form: it
+// converted w at every point of every tile, and 16 sums over 32 lanes one after the
+// other took 80 additions per warp.  The lanes now halve the number of sums they
+// hold at every step of the same tree (16 additions), and w is narrowed on the
+// integer ALUs (35 x 35 over 870001 FP32 points 458 -> 367 us, 21 x 21 215 -> 179, over 20001 26 -> 22; FP64
+// 250 thousand points and fewer 7 to 12 %; unrolled by four or eight the large FP32 cases take a fifth more,
+// and tiles of 5 to 8 are slower throughout).
 template <typename T, int TR>
 __global__ void __launch_bounds__(GTH) gram_tile_kernel(long long n, int a, int b, const T* __restrict__ A,
                                                         long long sa, const T* __restrict__ B, long long sb,
@@ -59,7 +88,7 @@ __global__ void __launch_bounds__(GTH) gram_tile_kernel(long long n, int a, int 
 #pragma unroll 2
   for (long long p = blockIdx.x * (long long)GTH + threadIdx.x; p < n; p += (long long)gridDim.x * GTH) {
     T av[TR], bv[TR];
-    const T wp = w ? T(w[p]) : T(1);
+    const T wp = w ? narrow(w[p], T()) : T(1);
 #pragma unroll
     for (int r = 0; r < TR; ++r) {
       av[r] = Ar[r] ? Ar[r][p] : T(0);
@@ -70,20 +99,36 @@ __global__ void __launch_bounds__(GTH) gram_tile_kernel(long long n, int a, int 
 #pragma unroll
       for (int c = 0; c < TR; ++c) acc[r][c] += av[r] * bv[c];
   }
-  // one output row at a time keeps the reduction's registers small
-  __shared__ double scratch[TR * (GTH / 32)];
-  double* pb = part + (long long)blockIdx.x * a * b;
+  // Sums over the lanes: step `off` pairs lanes off apart, the upper one of which goes on with the
+  // second half of the values, so each pair adds every value once; lane l ends with value `at`.
+  static_assert(TR * TR == 16, "four halvings");
+  constexpr int WARPS = GTH / 32;
+  __shared__ double scratch[WARPS][TR * TR];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double v[16];
 #pragma unroll
-  for (int r = 0; r < TR; ++r) {
-    double v[TR];
+  for (int e = 0; e < 16; ++e) v[e] = widen(acc[e / TR][e % TR]);
+  int at = 0;
 #pragma unroll
-    for (int c = 0; c < TR; ++c) v[c] = (double)acc[r][c];
-    block_sum<TR, GTH>(v, scratch);
-    if (threadIdx.x == 0 && i0 + r < a) {
+  for (int half = 8, off = 16; half >= 1; half /= 2, off /= 2) {
+    const bool up = lane & off;
+    at += up ? half : 0;
 #pragma unroll
-      for (int c = 0; c < TR; ++c)
-        if (j0 + c < b) pb[(long long)(i0 + r) * b + j0 + c] = v[c];
+    for (int e = 0; e < half; ++e) {
+      const double keep = up ? v[e + half] : v[e], send = up ? v[e] : v[e + half];
+      v[e] = keep + __shfl_xor_sync(0xffffffffu, send, off);
     }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  if (!(lane & 1)) scratch[warp][at] = v[0];
+  __syncthreads();
+  if (threadIdx.x < 16) {
+    const int e = threadIdx.x, r = i0 + e / TR, c = j0 + e % TR;
+    static_assert(WARPS == 8, "the tree over eight warps");
+    auto pair = [&](int q) { return scratch[q][e] + scratch[q + 4][e]; };
+    if (r < a && c < b)
+      part[(long long)blockIdx.x * a * b + (long long)r * b + c] =
+          (pair(0) + pair(2)) + (pair(1) + pair(3));
   }
 }
 
