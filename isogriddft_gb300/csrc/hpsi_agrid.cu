@@ -405,6 +405,15 @@ extern "C" int igd_hpsi_agrid(int dtype, int closure, int nx, int ny, int nz, co
                                          kscale, vscale, st);
     if (t >= 0) return t;
   }
+  // Blocks of rows of 129 to 160 points with the production closure: linear tiles, whose face work
+  // is dealt to a few threads, before the tiled kernel.  tiled / linear: 16 orbitals 160^3 397 / 344 us,
+  // 32 on 144^3 550 / 463, 4 on 132x100x148 52 / 49, 20 on 40x40x160 43 / 29; 8 on 176x160x180
+  // 239 / 266, 32 on 192^3 1167 / 1330; trial fix 160^3 234 / 365.
+  if (path == 0 && prod && dtype == IGD_F32 && nb > 1 && nz > 128 && nz <= 160) {
+    const int t = hpsi_agrid_lin_launch(dtype, closure, nx, ny, nz, coeffs, veff, psi, out, nb, orbital_stride, kscale,
+                                        vscale, st);
+    if (t >= 0) return t;
+  }
   if (path <= 1) {
     const int t = hpsi_agrid_tma_launch(dtype, closure, nx, ny, nz, coeffs, veff, psi, out, nb, orbital_stride, kscale,
                                         vscale, st);

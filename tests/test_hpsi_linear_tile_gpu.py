@@ -79,3 +79,32 @@ def test_linear_tile_kernels_against_the_oracle(shape, closure):
                         assert np.isnan(host[shift + o * st + n: shift + (o + 1) * st]).all()  # padding untouched
     finally:
         _lib.call("igd_hpsi_select", 0)
+
+
+@pytest.mark.parametrize("nz,linear", [(128, False), (132, True), (160, True), (164, False)])
+def test_production_blocks_of_long_rows(nz, linear):
+    """Rows of 129 to 160 points take the linear tiles, their neighbours the TMA kernels: the default
+    route equals the forced kernel to the bit and the tiled kernel to FP32 rounding."""
+
+    import torch
+
+    from isogriddft_gb300 import _lib, device, ops
+
+    geom = _geom((9, 11, nz))
+    dg = device.device_grid(geom)
+    g = torch.Generator(device="cuda").manual_seed(nz)
+    for nb in (2, 5):
+        psi = torch.randn(nb, dg.n, generator=g, device="cuda")
+        v = torch.randn(dg.n, generator=g, device="cuda")
+        got = {}
+        for path in (0, 1, 3):
+            _lib.call("igd_hpsi_select", path)
+            try:
+                got[path] = ops.hpsi_device(dg, psi, closure="production", veff=v).clone()
+            finally:
+                _lib.call("igd_hpsi_select", 0)
+        if linear:
+            assert torch.equal(got[0], got[3])
+        scale = float(got[1].abs().max())
+        assert float((got[0] - got[1]).abs().max()) <= 2e-5 * scale
+        assert float((got[3] - got[1]).abs().max()) <= 2e-5 * scale
