@@ -738,13 +738,14 @@ bool fused_poisson_enabled() { return g_poisson_path == 0; }
 // The operator of the fused path: out = -L psi with the dots (see hpsi_agrid_krylov), -1 when neither
 // kernel takes it.  Where both FP32 kernels do, small grids go to the linear-tile kernel: the
 // whole-row kernel's march has a latency of 14 us (27 us with rows of more than 128 points), whole-row
-// / linear-tile 48^3 14.3 / 8.1 us, 80^3 14.6 / 11.5, 68x84x92 14.8 / 12.6, 96^3 14.7 / 15.5, 128^3
-// 18.3 / 28.8; 64x64x192 27 / 17, 128x128x192 38 / 68.
+// / linear-tile 80^3 14.3 / 10.5 us, 88^3 14.5 / 12.2, 96^3 14.5 / 14.3, 104^3 14.9 / 17.2, 112^3
+// 16.0 / 20.1; 60x90x160 27.8 / 16.0, 100x100x144 27.0 / 21.5, 112x112x200 32.5 / 36.8.  Whole solves: 88x84x92
+// 16.6 / 14.8 ms, 96x92x88 no faster.
 template <typename T>
 int krylov_op(const Problem& P, const T* psi, T* out, const T* dot_y, double* acc, const int* skip, cudaStream_t q) {
   if constexpr (sizeof(T) == 4) {
     const float* c = static_cast<const float*>(P.c32);
-    const bool small = P.n <= (P.nz <= 128 ? 600000 : 1200000) && hpsi_agrid_lin_krylov_applies(P.nx, P.ny, P.nz);
+    const bool small = P.n <= (P.nz <= 128 ? 700000 : 1600000) && hpsi_agrid_lin_krylov_applies(P.nx, P.ny, P.nz);
     if (!small && hpsi_agrid_krylov_applies(P.nz, c)) {
       const int e = hpsi_agrid_krylov(P.nx, P.ny, P.nz, c, psi, out, -1.0, dot_y, acc, skip, q);
       if (e != -1) return e;
