@@ -740,12 +740,15 @@ bool fused_poisson_enabled() { return g_poisson_path == 0; }
 // whole-row kernel's march has a latency of 14 us (27 us with rows of more than 128 points), whole-row
 // / linear-tile 80^3 14.3 / 10.5 us, 88^3 14.5 / 12.2, 96^3 14.5 / 14.3, 104^3 14.9 / 17.2, 112^3
 // 16.0 / 20.1; 60x90x160 27.8 / 16.0, 100x100x144 27.0 / 21.5, 112x112x200 32.5 / 36.8.  Whole solves: 88x84x92
-// 16.6 / 14.8 ms, 96x92x88 no faster.
+// 16.6 / 14.8 ms, 96x92x88 no faster.  Below 50 thousand points the whole-row kernel stays, although slower
+// (14 and 8 us): the number of iterations varies with the order of the dot products, and of 40 solves on
+// 33x30x40 those on linear tiles took 74 to 85 iterations, on whole rows 71 to 78, unfused 68 to 75.
 template <typename T>
 int krylov_op(const Problem& P, const T* psi, T* out, const T* dot_y, double* acc, const int* skip, cudaStream_t q) {
   if constexpr (sizeof(T) == 4) {
     const float* c = static_cast<const float*>(P.c32);
-    const bool small = P.n <= (P.nz <= 128 ? 700000 : 1600000) && hpsi_agrid_lin_krylov_applies(P.nx, P.ny, P.nz);
+    const bool small = P.n >= 50000 && P.n <= (P.nz <= 128 ? 700000 : 1600000) &&
+                       hpsi_agrid_lin_krylov_applies(P.nx, P.ny, P.nz);
     if (!small && hpsi_agrid_krylov_applies(P.nz, c)) {
       const int e = hpsi_agrid_krylov(P.nx, P.ny, P.nz, c, psi, out, -1.0, dot_y, acc, skip, q);
       if (e != -1) return e;
