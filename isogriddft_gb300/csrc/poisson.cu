@@ -604,8 +604,10 @@ __device__ __forceinline__ void f_stop(FState* s, int j, int status) {
 // Iteration j, part 1: the stopping test on the previous iteration (k_next of
 // bicgstab<T>), then p = r + beta (p - omega v), beta = (rho_k / rho_{k-1})
 // (alpha_{k-1} / omega_{k-1}) (p = r on the first iteration); clears bank j+1.
+// bad_start: the status of a right-hand side with a NaN or an infinity.
 template <typename T, int E>
-__global__ void kf_p(long long nv, const T* __restrict__ r, T* __restrict__ p, const T* __restrict__ v, FState* s, int j, double rtol2, int maxit) {
+__global__ void kf_p(long long nv, const T* __restrict__ r, T* __restrict__ p, const T* __restrict__ v, FState* s, int j,
+                     double rtol2, int maxit, int bad_start) {
   // the scalar work (FP64 divisions, slow on GB300's FP64 pipe) once per block;
   // stop: -1 go on, -2 stopped before, else the status this iteration stops with
   __shared__ T sc[2];
@@ -621,7 +623,7 @@ __global__ void kf_p(long long nv, const T* __restrict__ r, T* __restrict__ p, c
       const int k = s->base + j;                // iterations completed
       const double rr = b1[B_RR];
       if (!isfinite(rr)) {
-        st = IGD_ERR_NONFINITE;
+        st = k > 0 ? IGD_ERR_NONFINITE : bad_start;
       } else if (k > 0 && rr <= rtol2 * s->bnorm2) {
         st = IGD_OK;
       } else {
@@ -780,12 +782,16 @@ int bicgstab_fused_run(const Problem& P, const T* f, T* x, double rtol, int maxi
   kf_init<T, E><<<nbv, PB, 0, st>>>(nv, P.nx, P.ny, P.nz, f, x, r, rh, p, v, S);
   kf_after_init<<<1, 1, 0, st>>>(S);
   const double rtol2 = rtol * rtol;
+  // the unfused iteration finds a right-hand side that is not finite in its first dot product and breaks
+  // down, which the entry points return; the whole-row FP32 solves stop as non-finite, and say so in info
+  const bool rows32 = sizeof(T) == 4 && E > 1 && hpsi_agrid_krylov_applies(P.nz, P.c32);
+  const int bad_start = rows32 ? IGD_ERR_NONFINITE : IGD_ERR_BREAKDOWN;
   constexpr int chunk = 8;  // a multiple of the 4 banks
   auto issue_chunk = [&](cudaStream_t q) -> int {
     kf_chunk_begin<<<1, 1, 0, q>>>(S, chunk);
     for (int j = 0; j < chunk; ++j) {
       double* bank = S->bank[j & 3];
-      kf_p<T, E><<<nbv, PB, 0, q>>>(nv, r, p, v, S, j, rtol2, maxit);
+      kf_p<T, E><<<nbv, PB, 0, q>>>(nv, r, p, v, S, j, rtol2, maxit, bad_start);
       int e = krylov_op<T>(P, p, v, rh, bank + B_RV, &S->done, q);
       if (e) return e < 0 ? IGD_ERR_ARG : e;
       kf_s<T, E><<<nbv, PB, 0, q>>>(nv, r, v, sv, S, j);

@@ -1,0 +1,57 @@
+"""The fused BiCGSTAB of the Poisson solve in every form that it takes, against the unfused one."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _grid(shape):
+    from isogriddft_gb300.config import H2_BENCHMARK_CASE
+    from isogriddft_gb300.device import device_grid
+    from isogriddft_gb300.grid import build_monitor_grid_for_case, build_two_peak_element_parameters
+
+    geom = build_monitor_grid_for_case(H2_BENCHMARK_CASE, shape=shape, box_half_extents=(8.0, 8.0, 10.0),
+                                       element_parameters=build_two_peak_element_parameters(("H",)), device=True)
+    return geom, device_grid(geom)
+
+
+def _solve(shape, c64, c32, f, precision, path=0, u=None, rtol=1e-10, maxit=3000):
+    """igd_poisson_solve, or igd_poisson_solve_from with u: return code, solution, info."""
+
+    import torch
+
+    from isogriddft_gb300 import _lib
+    from isogriddft_gb300.device import ptr, stream_ptr
+
+    n = int(np.prod(shape))
+    prec = _lib.IGD_PREC_FP64 if precision == "fp64" else _lib.IGD_PREC_MIXED
+    wsb = int(_lib.call("igd_poisson_workspace_bytes", prec, n))
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+    out = torch.empty(n, dtype=torch.float64, device="cuda") if u is None else u.clone()
+    info = np.zeros(6)
+    _lib.check(_lib.call("igd_poisson_select", path), "igd_poisson_select")
+    try:
+        code = _lib.call("igd_poisson_solve" if u is None else "igd_poisson_solve_from", _lib.IGD_GRID_MONITOR, prec,
+                         *shape, ptr(c64), ptr(c32), ptr(f), ptr(out), rtol, maxit, ptr(ws), wsb, info.ctypes.data,
+                         stream_ptr())
+    finally:
+        _lib.call("igd_poisson_select", 0)
+    return code, out, info
+
+
+@pytest.mark.parametrize("shape", [(11, 13, 15), (12, 14, 16)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_nonfinite_right_hand_side_is_a_breakdown(shape, bad):
+    """A right-hand side with a NaN or an infinity inside is refused with the unfused iteration's return code."""
+
+    import torch
+
+    from isogriddft_gb300 import _lib
+
+    geom, dg = _grid(shape)
+    f = torch.randn(shape, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    f[4, 5, 6] = bad
+    for path in (1, 0):
+        code, _, info = _solve(shape, dg.coeffs("fp64"), None, f.reshape(-1), "fp64", path)
+        assert code == _lib.IGD_ERR_BREAKDOWN and info[0] == 0 and info[2] == _lib.IGD_ERR_BREAKDOWN, (path, code, info)
