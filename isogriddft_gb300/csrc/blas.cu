@@ -34,10 +34,8 @@ inline bool gram64_split_pays(long long n, int a, int b) {
 }
 constexpr int GPT = 64;    // points per thread and block column (FP32 partial sums stay short)
 
-// FP64 <-> FP32 conversions on the integer ALUs (a converted value takes 16 clocks of the SM's FP64 pipe
-// per warp); zeros apart, values outside the normal range go through the instruction, in a call.
+// FP64 to FP32 on the integer ALUs, as widen (common.cuh).
 __device__ __noinline__ float narrow_slow(double x) { return (float)x; }
-__device__ __noinline__ double widen_slow(float x) { return (double)x; }
 __device__ __forceinline__ float narrow(double x) {  // to nearest, ties to even
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), e = (hi >> 20) & 0x7ffu;
   if (e - 897u > 253u) return narrow_slow(x);
@@ -48,13 +46,6 @@ __device__ __forceinline__ float narrow(double x) {  // to nearest, ties to even
 }
 __device__ __forceinline__ double narrow(double x, double) { return x; }
 __device__ __forceinline__ float narrow(double x, float) { return narrow(x); }
-__device__ __forceinline__ double widen(double x) { return x; }
-__device__ __forceinline__ double widen(float x) {
-  const unsigned u = __float_as_uint(x), e = (u >> 23) & 0xffu;
-  if ((u << 1) == 0u) return __hiloint2double((int)u, 0);
-  if (e - 1u > 253u) return widen_slow(x);
-  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
-}
 
 // Register-tiled tall-skinny Gram.  Block (x, y): tile y of TR x TR outputs
 // (rows i0.., columns j0..) over the points of column slice x; each thread

@@ -38,6 +38,18 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// ---------------------------------------------------------------- conversions
+// FP32 to FP64 on the integer ALUs (a converted value takes 16 clocks of the SM's FP64 pipe per warp);
+// zeros apart, values outside the normal range go through the instruction, in a call.
+static __device__ __noinline__ double widen_slow(float x) { return (double)x; }
+__device__ __forceinline__ double widen(double x) { return x; }
+__device__ __forceinline__ double widen(float x) {
+  const unsigned u = __float_as_uint(x), e = (u >> 23) & 0xffu;
+  if ((u << 1) == 0u) return __hiloint2double((int)u, 0);
+  if (e - 1u > 253u) return widen_slow(x);
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+
 // ---------------------------------------------------------------- reductions
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
@@ -115,11 +127,12 @@ int hpsi_agrid_lin_launch(int dtype, int closure, int nx, int ny, int nz, const 
                           const void* psi, void* out, int nb, long long ostride, double kscale, double vscale,
                           cudaStream_t st);
 
-// The linear-tile kernel as the Poisson operator of a Krylov solve, as hpsi_agrid_krylov below, in FP32 or
-// FP64 (acc[1] only when dot_y is null); -1 = not applicable.
+// The linear-tile kernel as the Poisson operator of a Krylov solve, as hpsi_agrid_krylov above, in FP32 or
+// FP64 (acc[1] only when dot_y is null); dots64: products and sums of FP32 dots in FP64.  -1 = not applicable.
 bool hpsi_agrid_lin_krylov_applies(int nx, int ny, int nz);
 int hpsi_agrid_lin_krylov(int dtype, int nx, int ny, int nz, const void* coeffs, const void* psi, void* out,
-                          double kscale, const void* dot_y, double* dot_acc, const int* skip, cudaStream_t st);
+                          double kscale, const void* dot_y, double* dot_acc, const int* skip, bool dots64,
+                          cudaStream_t st);
 
 // Whole-row z-vectorised fast path of igd_hpsi_agrid (hpsi_agrid_zvec.cu); -1 = not applicable.
 int hpsi_agrid_zvec_launch(int dtype, int closure, int nx, int ny, int nz, const void* coeffs, const void* veff,

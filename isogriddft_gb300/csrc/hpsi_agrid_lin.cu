@@ -423,7 +423,8 @@ __device__ __forceinline__ Cell<NB> cflux(float a1, Cell<NB> g1, float a2, Cell<
   return cfma(a3, g3, cfma(a1, g1, cmul(a2, g2)));
 }
 
-template <int NB, int PPT, bool PROD, bool KRY>
+// DOT: products and per-thread sums of the Krylov dots.
+template <int NB, int PPT, bool PROD, bool KRY, typename DOT = float>
 __global__ void __launch_bounds__(L32_NT, 1)
     hpsi_lin32_kernel(const float* __restrict__ coeffs, const float* __restrict__ veff, const float* __restrict__ psi,
                       float* __restrict__ out, const LinArgs a, float kscale, float vscale) {
@@ -445,7 +446,13 @@ __global__ void __launch_bounds__(L32_NT, 1)
   C zero;
 #pragma unroll
   for (int o = 0; o < NB; ++o) zero.v[o] = 0.f;
-  float d0 = 0.f, d1 = 0.f;  // Krylov dots: a few dozen terms per thread, FP64 across threads
+  DOT d0 = 0, d1 = 0;  // Krylov dots: a few dozen terms per thread, FP64 across threads
+  const auto dot = [](float x) -> DOT {
+    if constexpr (sizeof(DOT) == 8)
+      return widen(x);
+    else
+      return x;
+  };
   const int end = lin_bound(blockIdx.x + 1, a);
   for (int pos = lin_bound(blockIdx.x, a); pos < end;) {
     const LinSeg t = lin_seg(a, pos, end, NB);
@@ -540,10 +547,11 @@ __global__ void __launch_bounds__(L32_NT, 1)
         // faces of a Krylov vector stay zero; the dots then cover interior points only
         if (face[i] || op == 0 || op == nx - 1) val = zero;
         if (a.dot_y) {
-          d0 = fmaf(val.v[0], ld(static_cast<const float*>(a.dot_y), go), d0);
+          d0 = fma(dot(val.v[0]), dot(ld(static_cast<const float*>(a.dot_y), go)), d0);
         } else {
-          d0 = fmaf(val.v[0], ps.v[0], d0);
-          d1 = fmaf(val.v[0], val.v[0], d1);
+          const DOT v0 = dot(val.v[0]);
+          d0 = fma(v0, dot(ps.v[0]), d0);
+          d1 = fma(v0, v0, d1);
         }
       }
 #pragma unroll
@@ -782,7 +790,7 @@ int lin64_v(const double* c, const double* v, const double* p, double* o, int nx
   return lin64_launch<PROD, false, true>(c, v, p, o, nx, ny, nz, nb, ostride, kscale, st);
 }
 
-template <int NB, int PPT, bool PROD, bool KRY>
+template <int NB, int PPT, bool PROD, bool KRY, typename DOT = float>
 int lin32_launch(const float* coeffs, const float* veff, const float* psi, float* out, int nx, int ny, int nz, int nb,
                  long long ostride, double kscale, double vscale, cudaStream_t st, const float* dot_y = nullptr,
                  double* dot_acc = nullptr, const int* skip = nullptr) {
@@ -793,7 +801,7 @@ int lin32_launch(const float* coeffs, const float* veff, const float* psi, float
                                      1250.0, 4.5, 1.0});
   if (p.tiles == 0) return -1;
   const size_t smem = lin32_cells<NB>(p.oymax, nz) * sizeof(float) * NB;
-  auto kern = hpsi_lin32_kernel<NB, PPT, PROD, KRY>;
+  auto kern = hpsi_lin32_kernel<NB, PPT, PROD, KRY, DOT>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != IGD_OK) return IGD_ERR_CUDA;
   const LinArgs a = lin_args(p, nx, ny, nz, nb, ostride, groups, dot_y, dot_acc, skip);
   kern<<<(unsigned)p.ctas, L32_NT, smem, st>>>(coeffs, veff, psi, out, a, (float)kscale, (float)vscale);
@@ -849,7 +857,8 @@ int hpsi_agrid_lin_launch(int dtype, int closure, int nx, int ny, int nz, const 
 bool hpsi_agrid_lin_krylov_applies(int nx, int ny, int nz) { return lin_ok(nx, ny, nz); }
 
 int hpsi_agrid_lin_krylov(int dtype, int nx, int ny, int nz, const void* coeffs, const void* psi, void* out,
-                          double kscale, const void* dot_y, double* dot_acc, const int* skip, cudaStream_t st) {
+                          double kscale, const void* dot_y, double* dot_acc, const int* skip, bool dots64,
+                          cudaStream_t st) {
   if (!lin_ok(nx, ny, nz) || !dot_acc) return -1;
   const long long n = (long long)nx * ny * nz;
   if (dtype == IGD_F64)
@@ -859,9 +868,13 @@ int hpsi_agrid_lin_krylov(int dtype, int nx, int ny, int nz, const void* coeffs,
   const float *c = static_cast<const float*>(coeffs), *p = static_cast<const float*>(psi),
               *y = static_cast<const float*>(dot_y);
   float* o = static_cast<float*>(out);
-  if (nz > L32_NT * 2 / 5)
-    return lin32_launch<1, 3, true, true>(c, nullptr, p, o, nx, ny, nz, 1, n, kscale, 0.0, st, y, dot_acc, skip);
-  return lin32_launch<1, 2, true, true>(c, nullptr, p, o, nx, ny, nz, 1, n, kscale, 0.0, st, y, dot_acc, skip);
+  const auto run = [&](auto dot) {
+    using D = decltype(dot);
+    if (nz > L32_NT * 2 / 5)
+      return lin32_launch<1, 3, true, true, D>(c, nullptr, p, o, nx, ny, nz, 1, n, kscale, 0.0, st, y, dot_acc, skip);
+    return lin32_launch<1, 2, true, true, D>(c, nullptr, p, o, nx, ny, nz, 1, n, kscale, 0.0, st, y, dot_acc, skip);
+  };
+  return dots64 ? run(0.0) : run(0.f);
 }
 
 }  // namespace igd

@@ -10,6 +10,7 @@
 // field whose face entries are kept at zero.
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -524,8 +525,9 @@ int bicgstab(const Problem& P, const T* f, T* x, double rtol, int maxit, unsigne
 // and its first kernel clears bank j+1 (chunks are a multiple of 4 long).
 // Per iteration: p update, v = A p (+ r^.v), s update, t = A s (+ t.s, t.t),
 // x / r update (+ r.r, r^.r): five launches, no single-thread kernels.
-// The arithmetic is the same BiCGSTAB as bicgstab<T> above.  Vectors move in 16-byte pieces where
-// n and the pointers allow (E values), else value by value (odd grids).
+// The recurrences are those of bicgstab<T> above, and so is the precision of the dot products: vectors
+// move in 16-byte pieces (E values) where nz and the pointers allow, with FP32 products and per-thread
+// sums in an FP32 solve, else value by value (odd grids) with every product and sum in FP64.
 enum { B_RV = 0, B_VV = 1, B_TS = 2, B_TT = 3, B_RR = 4, B_RHR = 5, B_N = 6 };
 struct FState {
   double bnorm2;
@@ -533,6 +535,18 @@ struct FState {
   int done, stop, status, chunk, base, pad[3];
 };
 static_assert(sizeof(FState) <= 256, "FState must fit the 256-byte state slot of the Krylov workspace");
+
+// Products and per-thread sums of the dot products.  FP64 ones on odd grids cost 55.6 us an iteration
+// for 51.7 with FP32 (67x67x81; 101x97x99 79.8 and 70.8), with the conversion instruction 59.7 (92.1).
+template <typename T, int E>
+using DotT = std::conditional_t<E == 1, double, T>;
+template <typename D, typename T>
+__device__ __forceinline__ D dot_value(T x) {
+  if constexpr (sizeof(D) > sizeof(T))
+    return widen(x);
+  else
+    return x;
+}
 
 template <typename T, int E>
 __device__ __forceinline__ void fld(const T* __restrict__ p, long long v, T (&o)[E]) {
@@ -555,7 +569,7 @@ __global__ void kf_state_init(FState* s) { memset(s, 0, sizeof(FState)); }
 template <typename T, int E>
 __global__ void kf_init(long long nv, int nx, int ny, int nz, const T* __restrict__ f, T* x, T* r, T* rh, T* p, T* v,
                         FState* s) {
-  T a = T(0);
+  DotT<T, E> a = 0;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nv; q += (long long)gridDim.x * blockDim.x) {
     T ff[E], z[E];
     fld<T, E>(f, q, ff);
@@ -568,7 +582,8 @@ __global__ void kf_init(long long nv, int nx, int ny, int nz, const T* __restric
     for (int e = 0; e < E; ++e) {
       ff[e] = (fb >> e) & 1u ? T(0) : ff[e];
       z[e] = T(0);
-      a += ff[e] * ff[e];
+      const DotT<T, E> d = dot_value<DotT<T, E>>(ff[e]);
+      a += d * d;
     }
     fst<T, E>(r, q, ff);
     fst<T, E>(rh, q, ff);
@@ -712,7 +727,8 @@ __global__ void kf_xr(long long nv, T* __restrict__ x, T* __restrict__ r, const 
   __syncthreads();
   if (!go) return;
   const T al = sc[0], om = sc[1];
-  T a = T(0), b = T(0);
+  using D = DotT<T, E>;
+  D a = 0, b = 0;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nv; q += (long long)gridDim.x * blockDim.x) {
     T xx[E], pp[E], ss[E], tv[E], hh[E], ro[E];
     fld<T, E>(x, q, xx);
@@ -724,8 +740,9 @@ __global__ void kf_xr(long long nv, T* __restrict__ x, T* __restrict__ r, const 
     for (int e = 0; e < E; ++e) {
       xx[e] = xx[e] + al * pp[e] + om * ss[e];
       ro[e] = ss[e] - om * tv[e];
-      a += ro[e] * ro[e];
-      b += hh[e] * ro[e];
+      const D d = dot_value<D>(ro[e]);
+      a += d * d;
+      b += dot_value<D>(hh[e]) * d;
     }
     fst<T, E>(x, q, xx);
     fst<T, E>(r, q, ro);
@@ -745,9 +762,12 @@ bool fused_poisson_enabled() { return g_poisson_path == 0; }
 // 16.6 / 14.8 ms, 96x92x88 no faster.  Below 50 thousand points the whole-row kernel stays, although slower
 // (14 and 8 us): the number of iterations varies with the order of the dot products, and of 40 solves on
 // 33x30x40 those on linear tiles took 74 to 85 iterations, on whole rows 71 to 78, unfused 68 to 75.
-template <typename T>
+// Vectors of single values (E = 1) have their dots formed in FP64.
+template <typename T, int E>
 int krylov_op(const Problem& P, const T* psi, T* out, const T* dot_y, double* acc, const int* skip, cudaStream_t q) {
-  if constexpr (sizeof(T) == 4) {
+  if constexpr (sizeof(T) == 4 && E == 1) {
+    return hpsi_agrid_lin_krylov(IGD_F32, P.nx, P.ny, P.nz, P.c32, psi, out, -1.0, dot_y, acc, skip, true, q);
+  } else if constexpr (sizeof(T) == 4) {
     const float* c = static_cast<const float*>(P.c32);
     const bool small = P.n >= 50000 && P.n <= (P.nz <= 128 ? 700000 : 1600000) &&
                        hpsi_agrid_lin_krylov_applies(P.nx, P.ny, P.nz);
@@ -755,9 +775,9 @@ int krylov_op(const Problem& P, const T* psi, T* out, const T* dot_y, double* ac
       const int e = hpsi_agrid_krylov(P.nx, P.ny, P.nz, c, psi, out, -1.0, dot_y, acc, skip, q);
       if (e != -1) return e;
     }
-    return hpsi_agrid_lin_krylov(IGD_F32, P.nx, P.ny, P.nz, c, psi, out, -1.0, dot_y, acc, skip, q);
+    return hpsi_agrid_lin_krylov(IGD_F32, P.nx, P.ny, P.nz, c, psi, out, -1.0, dot_y, acc, skip, false, q);
   } else {
-    return hpsi_agrid_lin_krylov(IGD_F64, P.nx, P.ny, P.nz, P.c64, psi, out, -1.0, dot_y, acc, skip, q);
+    return hpsi_agrid_lin_krylov(IGD_F64, P.nx, P.ny, P.nz, P.c64, psi, out, -1.0, dot_y, acc, skip, true, q);
   }
 }
 
@@ -792,10 +812,10 @@ int bicgstab_fused_run(const Problem& P, const T* f, T* x, double rtol, int maxi
     for (int j = 0; j < chunk; ++j) {
       double* bank = S->bank[j & 3];
       kf_p<T, E><<<nbv, PB, 0, q>>>(nv, r, p, v, S, j, rtol2, maxit, bad_start);
-      int e = krylov_op<T>(P, p, v, rh, bank + B_RV, &S->done, q);
+      int e = krylov_op<T, E>(P, p, v, rh, bank + B_RV, &S->done, q);
       if (e) return e < 0 ? IGD_ERR_ARG : e;
       kf_s<T, E><<<nbv, PB, 0, q>>>(nv, r, v, sv, S, j);
-      e = krylov_op<T>(P, sv, t, nullptr, bank + B_TS, &S->done, q);
+      e = krylov_op<T, E>(P, sv, t, nullptr, bank + B_TS, &S->done, q);
       if (e) return e < 0 ? IGD_ERR_ARG : e;
       kf_xr<T, E><<<nbv, PB, 0, q>>>(nv, x, r, p, sv, t, rh, S, j);
     }

@@ -55,3 +55,28 @@ def test_nonfinite_right_hand_side_is_a_breakdown(shape, bad):
     for path in (1, 0):
         code, _, info = _solve(shape, dg.coeffs("fp64"), None, f.reshape(-1), "fp64", path)
         assert code == _lib.IGD_ERR_BREAKDOWN and info[0] == 0 and info[2] == _lib.IGD_ERR_BREAKDOWN, (path, code, info)
+
+
+@pytest.mark.parametrize("shape", [(11, 13, 15), (7, 9, 211)])
+def test_ragged_mixed_solve_sums_dots_in_fp64(shape):
+    """Rows that are no multiple of four points: the FP32 iteration forms the products of its dot products in FP64, so
+    an operator of 1e24 times the size (t.t beyond FP32's range) gives the same solution, scaled."""
+
+    import torch
+
+    from isogriddft_gb300 import _lib
+
+    geom, dg = _grid(shape)
+    n = int(np.prod(shape))
+    f = torch.randn(n, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(4))
+    c64, c32 = dg.coeffs("fp64").reshape(7, n), dg.coeffs("fp32").reshape(7, n)
+    scale = 2.0**80
+    s64, s32 = c64.clone(), c32.clone()
+    s64[6] *= scale
+    s32[6] *= scale
+    sols = [_solve(shape, a, b, f, "mixed") for a, b in ((c64, c32), (s64, s32))]
+    for code, _, info in sols:
+        assert code == _lib.IGD_OK and info[1] <= 1e-10, (code, info)
+    # two solutions with relative residuals of 1e-10 each
+    u, v = sols[0][1], sols[1][1] * scale
+    assert float((u - v).norm() / u.norm()) < 1e-7
