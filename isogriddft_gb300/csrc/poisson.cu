@@ -781,12 +781,20 @@ int krylov_op(const Problem& P, const T* psi, T* out, const T* dot_y, double* ac
   }
 }
 
-// The fused path applies: a monitor grid whose rows a Krylov-mode operator takes.
+// 16-byte pieces neither cross a grid row nor break the alignment of any vector.
 template <typename T>
-bool fused_applies(const Problem& P) {
+bool pieces_ok(const Problem& P, const T* f, const T* x, const unsigned char* ws) {
+  const auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+  return P.nz % VecT<T>::E == 0 && al16(f) && al16(x) && al16(ws);
+}
+
+// The fused path applies: a monitor grid that a Krylov-mode operator takes, the linear-tile kernel (which
+// any vectors suit) or, with 16-byte pieces, the whole-row kernel.
+template <typename T>
+bool fused_applies(const Problem& P, const T* f, const T* x, const unsigned char* ws) {
   if (P.kind != IGD_GRID_MONITOR || (sizeof(T) == 4 && !P.c32)) return false;
-  if (sizeof(T) == 4 && hpsi_agrid_krylov_applies(P.nz, P.c32)) return true;
-  return hpsi_agrid_lin_krylov_applies(P.nx, P.ny, P.nz);
+  if (hpsi_agrid_lin_krylov_applies(P.nx, P.ny, P.nz)) return true;
+  return sizeof(T) == 4 && hpsi_agrid_krylov_applies(P.nz, P.c32) && pieces_ok<T>(P, f, x, ws);
 }
 
 template <typename T, int E>
@@ -865,14 +873,11 @@ int bicgstab_fused_run(const Problem& P, const T* f, T* x, double rtol, int maxi
   return h.status == IGD_ERR_NOT_CONVERGED ? IGD_OK : h.status;  // non-convergence is reported via rel
 }
 
-// Pieces of 16 bytes when they neither cross a grid row nor break the alignment of any vector.
 template <typename T>
 int bicgstab_fused(const Problem& P, const T* f, T* x, double rtol, int maxit, unsigned char* ws, int* iters,
                    double* rel, double* bnorm = nullptr) {
   constexpr int E = VecT<T>::E;
-  const auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
-  if (P.nz % E == 0 && al16(f) && al16(x) && al16(ws))
-    return bicgstab_fused_run<T, E>(P, f, x, rtol, maxit, ws, iters, rel, bnorm);
+  if (pieces_ok<T>(P, f, x, ws)) return bicgstab_fused_run<T, E>(P, f, x, rtol, maxit, ws, iters, rel, bnorm);
   return bicgstab_fused_run<T, 1>(P, f, x, rtol, maxit, ws, iters, rel, bnorm);
 }
 
@@ -958,7 +963,7 @@ static int poisson_solve(int grid_kind, int precision, int nx, int ny, int nz, c
   unsigned char* kry = w + 2 * (size_t)n * sizeof(double) + 256;
   int iters = 0, rounds = 0, status = IGD_OK;
   double rel = 0.0, rnorm = 0.0, rmax = 0.0, fnorm = 0.0;
-  const bool fused64 = precision == IGD_PREC_FP64 && fused_poisson_enabled() && fused_applies<double>(P);
+  const bool fused64 = precision == IGD_PREC_FP64 && fused_poisson_enabled() && fused_applies<double>(P, f, u, kry);
   if (precision == IGD_PREC_FP64 && !from_u) {
     status = fused64 ? bicgstab_fused<double>(P, f, u, rtol, max_iterations, kry, &iters, &rel, &fnorm)
                      : bicgstab<double>(P, f, u, rtol, max_iterations, kry, &iters, &rel, &fnorm);
@@ -980,7 +985,7 @@ static int poisson_solve(int grid_kind, int precision, int nx, int ny, int nz, c
     float* r32 = reinterpret_cast<float*>(kry);
     float* d32 = r32 + n;
     unsigned char* k32 = kry + 2 * (size_t)n * sizeof(float);
-    const bool fused = fused_poisson_enabled() && fused_applies<float>(P);
+    const bool fused = fused_poisson_enabled() && fused_applies<float>(P, r32, d32, k32);
     int e;
     if (from_u) {
       e = rhs_norm(P, f, Au, res, scal, &fnorm);

@@ -80,3 +80,30 @@ def test_ragged_mixed_solve_sums_dots_in_fp64(shape):
     # two solutions with relative residuals of 1e-10 each
     u, v = sols[0][1], sols[1][1] * scale
     assert float((u - v).norm() / u.norm()) < 1e-7
+
+
+def test_large_grid_with_a_workspace_aligned_to_a_double():
+    """More points than 32-bit offsets reach and vectors without 16-byte alignment: neither fused operator takes the
+    grid, so the unfused iteration does."""
+
+    import torch
+
+    from isogriddft_gb300 import _lib
+    from isogriddft_gb300.device import ptr, stream_ptr
+
+    shape = (800, 800, 248)
+    n = int(np.prod(shape))
+    assert 28 * n >= 1 << 32
+    c64 = torch.zeros((7, n), dtype=torch.float64, device="cuda")
+    for i in (0, 1, 2, 6):
+        c64[i] = 1.0
+    c32 = c64.float()
+    f = torch.zeros(n, dtype=torch.float64, device="cuda")
+    f[(400 * 800 + 400) * 248 + 124] = 1.0  # an interior point
+    u = torch.empty_like(f)
+    wsb = int(_lib.call("igd_poisson_workspace_bytes", _lib.IGD_PREC_MIXED, n))
+    buf = torch.empty(wsb + 16, dtype=torch.uint8, device="cuda")
+    info = np.zeros(6)
+    code = _lib.call("igd_poisson_solve", _lib.IGD_GRID_MONITOR, _lib.IGD_PREC_MIXED, *shape, ptr(c64), ptr(c32),
+                     ptr(f), ptr(u), 1e-2, 1, ptr(buf) + 8, wsb, info.ctypes.data, stream_ptr())
+    assert code == _lib.IGD_OK and info[0] == 1 and 0.0 < info[1] < 1.0, (code, info)
