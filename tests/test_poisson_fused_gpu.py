@@ -107,3 +107,51 @@ def test_large_grid_with_a_workspace_aligned_to_a_double():
     code = _lib.call("igd_poisson_solve", _lib.IGD_GRID_MONITOR, _lib.IGD_PREC_MIXED, *shape, ptr(c64), ptr(c32),
                      ptr(f), ptr(u), 1e-2, 1, ptr(buf) + 8, wsb, info.ctypes.data, stream_ptr())
     assert code == _lib.IGD_OK and info[0] == 1 and 0.0 < info[1] < 1.0, (code, info)
+
+
+# E = 2, odd rows (E = 1), rows of 205 to 256 points of either parity, the smallest grid; from_u: a warm start
+@pytest.mark.parametrize("shape", [(20, 18, 26), (21, 22, 23), (9, 11, 205), (8, 10, 256), (3, 3, 3)])
+@pytest.mark.parametrize("from_u", [False, True])
+def test_fused_fp64_iteration_matches_unfused(shape, from_u):
+    """FP64: both iterations meet the stopping rule and give the same solution."""
+
+    import torch
+
+    from isogriddft_gb300 import _lib
+
+    geom, dg = _grid(shape)
+    n = int(np.prod(shape))
+    g = torch.Generator("cuda").manual_seed(5)
+    f = torch.randn(n, dtype=torch.float64, device="cuda", generator=g)
+    u0 = None
+    if from_u:
+        u0 = torch.zeros(shape, dtype=torch.float64, device="cuda")
+        u0[1:-1, 1:-1, 1:-1] = torch.randn([m - 2 for m in shape], dtype=torch.float64, device="cuda", generator=g)
+        u0 = u0.reshape(-1)
+    sols = [_solve(shape, dg.coeffs("fp64"), None, f, "fp64", path, u0, rtol=1e-11) for path in (0, 1)]
+    for code, u, info in sols:
+        assert code == _lib.IGD_OK and info[1] <= 2e-11, (code, info)  # the recomputed residual, not the recursion's
+        q = u.reshape(shape)
+        for face in (q[0], q[-1], q[:, 0], q[:, -1], q[:, :, 0], q[:, :, -1]):
+            assert not face.any()
+    a, b = (s[1] for s in sols)
+    assert float((a - b).norm() / b.norm()) < 1e-8
+
+
+# rows of 205 to 256 points: no multiple of four, and of eight with at least 50 thousand points (both linear tiles)
+@pytest.mark.parametrize("shape", [(9, 11, 211), (16, 16, 208)])
+def test_fused_mixed_iteration_on_long_rows(shape):
+    """Mixed precision on rows that the linear-tile operator takes with three points per thread."""
+
+    import torch
+
+    from isogriddft_gb300 import _lib
+
+    geom, dg = _grid(shape)
+    f = torch.randn(int(np.prod(shape)), dtype=torch.float64, device="cuda",
+                    generator=torch.Generator("cuda").manual_seed(6))
+    sols = [_solve(shape, dg.coeffs("fp64"), dg.coeffs("fp32"), f, "mixed", path) for path in (0, 1)]
+    for code, _, info in sols:
+        assert code == _lib.IGD_OK and info[1] <= 1e-10, (code, info)
+    a, b = (s[1] for s in sols)
+    assert float((a - b).norm() / b.norm()) < 1e-7
