@@ -819,13 +819,10 @@ extern "C" int igd_block_gram(int dtype, long long n, int a, const void* A, long
     if (r != -1) return r;
   }
   if (dtype == IGD_F64 && (path == 4 || (path == 0 && gram64_split_pays(n, a, b)))) {
-    const int r = gram64_split_launch(n, a, static_cast<const double*>(A), sa, b, static_cast<const double*>(B), sb, w,
-                                      out, accumulate, reinterpret_cast<longlong2*>(part), gram_blocks(n),
-                                      reinterpret_cast<int*>(part + 2LL * gram_blocks(n) * a * b), st);
-    if (r != -1) {
-      g_gram_last = 4;
-      return r;
-    }
+    g_gram_last = 4;
+    return gram64_split_launch(n, a, static_cast<const double*>(A), sa, b, static_cast<const double*>(B), sb, w, out,
+                               accumulate, reinterpret_cast<longlong2*>(part), gram_blocks(n),
+                               reinterpret_cast<int*>(part + 2LL * gram_blocks(n) * a * b), st);
   }
   // the pipelined kernel when rows are 16-byte aligned and outputs <= 64 x 64, else the register-tiled one
   const int e = path == 3 ? -1

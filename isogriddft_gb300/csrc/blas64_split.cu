@@ -306,24 +306,31 @@ __global__ void gram64_reduce_kernel(int nblocks, long long n, int a, const doub
 
 }  // namespace
 
-// Windows per warp stay below 120 (an int32 level sum takes 127 windows of at most 2^24).
+// At most 120 windows per warp (an int32 level sum takes 127 windows of at most 2^24): more than max_blocks CTAs
+// can take go in pieces, each with its own row exponents, added up in the output.  9.5 million points:
+// two pieces.
 int gram64_split_launch(long long n, int a, const double* A, long long sa, int b, const double* B, long long sb,
                         const double* w, double* out, int accumulate, longlong2* part, int max_blocks, int* emax,
                         cudaStream_t st) {
+  constexpr long long MOST = 120, WINDOW = 32 * GW;
   const int sms = device_sm_count();
   const int ty = (a + 15) / 16, tz = (b + 8 * GNT - 1) / (8 * GNT);
-  const long long windows = (n + 32 * GW - 1) / (32 * GW);
-  long long grid = std::min<long long>(windows, std::max(1, 2 * sms / (ty * tz)));
-  grid = std::min<long long>(std::max(grid, (windows + 119) / 120), max_blocks);
-  if (windows > 120 * grid) return -1;
   const int sym = A == B && sa == sb && a == b;
-  if (cudaMemsetAsync(emax, 0, sizeof(int) * (a + b), st) != cudaSuccess) return IGD_ERR_CUDA;
-  row_exponent_kernel<<<dim3((unsigned)((n + ETH * EU - 1) / (ETH * EU)), (a + b + ER - 1) / ER), ETH, 0, st>>>(
-      n, a, A, sa, b, B, sb, w, emax);
+  const long long windows = (n + WINDOW - 1) / WINDOW, pieces = (windows + MOST * max_blocks - 1) / (MOST * max_blocks);
+  const long long step = (windows + pieces - 1) / pieces * WINDOW;  // points of a piece
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(gram64_kernel), GSMEM) != IGD_OK) return IGD_ERR_CUDA;
-  gram64_kernel<<<dim3((unsigned)grid, ty, tz), 32 * GW, GSMEM, st>>>(n, a, A, sa, b, B, sb, w, emax, sym, part);
-  gram64_reduce_kernel<<<std::min((a * b * 32 + 255) / 256, 1024), 256, 0, st>>>((int)grid, n, a, A, sa, b, B, sb, w,
-                                                                               emax, sym, part, out, accumulate);
+  for (long long p0 = 0; p0 < n; p0 += step) {
+    const long long m = std::min(step, n - p0), mw = (m + WINDOW - 1) / WINDOW;
+    const double *pa = A + p0, *pb = B + p0, *pw = w ? w + p0 : nullptr;
+    const long long want = std::min<long long>(mw, std::max<long long>(1, 2LL * sms / ((long long)ty * tz)));
+    const int grid = (int)std::min<long long>(std::max(want, (mw + MOST - 1) / MOST), max_blocks);
+    if (cudaMemsetAsync(emax, 0, sizeof(int) * (a + b), st) != cudaSuccess) return IGD_ERR_CUDA;
+    row_exponent_kernel<<<dim3((unsigned)((m + ETH * EU - 1) / (ETH * EU)), (a + b + ER - 1) / ER), ETH, 0, st>>>(
+        m, a, pa, sa, b, pb, sb, pw, emax);
+    gram64_kernel<<<dim3((unsigned)grid, ty, tz), 32 * GW, GSMEM, st>>>(m, a, pa, sa, b, pb, sb, pw, emax, sym, part);
+    gram64_reduce_kernel<<<(int)std::min<long long>(((long long)a * b + 7) / 8, 1024), 256, 0, st>>>(
+        grid, m, a, pa, sa, b, pb, sb, pw, emax, sym, part, out, accumulate || p0 > 0);
+  }
   return launch_status();
 }
 
