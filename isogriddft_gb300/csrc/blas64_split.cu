@@ -266,8 +266,8 @@ __global__ void __launch_bounds__(32 * GW, 2)
 }
 
 // out[i][j] (+)= sum over CTAs, one warp per output; a symmetric product takes its lower triangle
-// from the upper.  Outputs whose row or column holds an infinity or a NaN (or may overflow) are
-// summed plainly in FP64 here.
+// from the upper.  Outputs whose row or column holds an infinity or a NaN (or may overflow, in the
+// mirrored product too) are summed plainly in FP64 here.
 __global__ void gram64_reduce_kernel(int nblocks, long long n, int a, const double* __restrict__ A, long long sa, int b,
                                      const double* __restrict__ B, long long sb, const double* __restrict__ w,
                                      const int* __restrict__ emax, int sym, const longlong2* __restrict__ part,
@@ -277,7 +277,8 @@ __global__ void gram64_reduce_kernel(int nblocks, long long n, int a, const doub
   for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < ab; e += (gridDim.x * blockDim.x) >> 5) {
     const int i = e / b, j = e - i * b;
     double v = 0.0;
-    if (emax[i] >= 0x7ff || emax[a + j] >= 0x7ff) {
+    const bool special = emax[i] >= 0x7ff || emax[a + j] >= 0x7ff || (sym && (emax[j] >= 0x7ff || emax[a + i] >= 0x7ff));
+    if (special) {
       for (long long p = lane; p < n; p += 32)
         v += A[(long long)i * sa + p] * (B[(long long)j * sb + p] * (w ? w[p] : 1.0));
     } else {
@@ -298,7 +299,7 @@ __global__ void gram64_reduce_kernel(int nblocks, long long n, int a, const doub
         v = join(q.x, q.y, ei + ej - 2166 + 63);
       }
     }
-    if (emax[i] >= 0x7ff || emax[a + j] >= 0x7ff)
+    if (special)
       for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
     if (lane == 0) out[e] = accumulate ? out[e] + v : v;
   }

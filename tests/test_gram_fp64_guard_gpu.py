@@ -46,3 +46,24 @@ def test_split_gram_above_nine_million_points():
     assert last == 4 and np.all(np.abs(got - plain) <= 2.0**-44 * scale.cpu().numpy())
     _, more, _ = _gram(A, B, w, 4, out=torch.full((3, 2), 1.0, dtype=torch.float64, device="cuda"))
     assert np.all(np.abs(more - 1.0 - got) <= 2.0**-50 * np.abs(got) + 2.0**-50)
+
+
+def test_self_gram_with_an_overflowing_product():
+    """w x of one row overflows while x is finite: outputs of that row and column as the plain kernel gives them."""
+
+    import torch
+
+    n, a = 4000, 19
+    g = torch.Generator("cuda").manual_seed(1)
+    X = torch.randn((a, n), dtype=torch.float64, device="cuda", generator=g)
+    w = torch.rand(n, dtype=torch.float64, device="cuda", generator=g) + 1e-3
+    p = 777
+    w[p] = 1e150
+    X[:, p] = 1e-200
+    X[7, p] = 1e200
+    (_, got, last), (_, plain, _) = _gram(X, X, w, 4), _gram(X, X, w, 3)
+    assert last == 4
+    assert np.array_equal(np.isnan(got), np.isnan(plain)) and np.array_equal(np.isinf(got), np.isinf(plain))
+    fine = np.isfinite(plain)
+    assert fine[7].sum() == a - 1 and not fine[:, 7].any()  # (i, 7) multiplies the infinity, (7, j) does not
+    assert np.all(np.abs(got - plain)[fine] <= 1e-12 * np.abs(plain)[fine] + 1e-9)
