@@ -222,6 +222,8 @@ int igd_density_residual2(long long n, const double* up_in, const double* dn_in,
  * weighted_overlap_matrix (ks/eigensolver.py:246-272) and
  * _weighted_overlap_columns (ks/eigensolver_jax.py:105); rotation replaces the
  * basis @ coeffs products and two-part compressions (eigensolver_jax.py:178-251). */
+/* The workspace is aligned to a double at least; with 16-byte alignment FP64
+ * products on large grids use the tensor pipe, else CUDA cores. */
 long long igd_block_gram_workspace_bytes(long long n, int a, int b);
 /* out (a x b FP64) [+]= A diag(w) B^T (w may be NULL); FP64 accumulation.
  * FP32 blocks of up to 64 x 64 outputs with 16-byte aligned rows run on the

@@ -785,13 +785,17 @@ extern "C" int igd_gram_select(int path) {
   return IGD_OK;
 }
 
+// Per-block partials of the plain kernels and the FP32 tensor-core one; the workspace that every call needs.
+static long long gram_plain_bytes(long long n, int a, int b) {
+  return (long long)gram_blocks(n) * a * b * (long long)sizeof(double);
+}
+
 // Kernel used by the calling thread's last igd_block_gram (0 before any call).
 extern "C" int igd_gram_last_path(void) { return g_gram_last; }
 
 extern "C" long long igd_block_gram_workspace_bytes(long long n, int a, int b) {
   if (n <= 0 || a <= 0 || b <= 0) return -1;
-  // per-block partials (pairs in the FP64 splitting kernel), and that kernel's row exponents
-  return (2LL * gram_blocks(n) * a * b + (a + b + 1) / 2) * (long long)sizeof(double);
+  return gram_plain_bytes(n, a, b) + gram64_split_bytes(1, a, b);
 }
 
 // out (a x b, FP64, row-major) [+]= A W B^T for row-major blocks A (a x n, row
@@ -800,7 +804,7 @@ extern "C" int igd_block_gram(int dtype, long long n, int a, const void* A, long
                               long long sb, const double* w, double* out, int accumulate, void* workspace,
                               long long workspace_bytes, void* stream) {
   if (n <= 0 || a <= 0 || b <= 0 || !A || !B || !out || !workspace) return IGD_ERR_ARG;
-  if (workspace_bytes < igd_block_gram_workspace_bytes(n, a, b)) return IGD_ERR_ARG;
+  if (workspace_bytes < gram_plain_bytes(n, a, b)) return IGD_ERR_ARG;
   if (dtype != IGD_F32 && dtype != IGD_F64) return IGD_ERR_DTYPE;
   cudaStream_t st = as_stream(stream);
   int nb = gram_pipe_blocks(n);
@@ -818,11 +822,16 @@ extern "C" int igd_block_gram(int dtype, long long n, int a, const void* A, long
     }
     if (r != -1) return r;
   }
-  if (dtype == IGD_F64 && (path == 4 || (path == 0 && gram64_split_pays(n, a, b)))) {
-    g_gram_last = 4;
-    return gram64_split_launch(n, a, static_cast<const double*>(A), sa, b, static_cast<const double*>(B), sb, w, out,
-                               accumulate, reinterpret_cast<longlong2*>(part), gram_blocks(n),
-                               reinterpret_cast<int*>(part + 2LL * gram_blocks(n) * a * b), st);
+  // FP64: exact splitting, in a workspace that is aligned for its pairs of integers and holds at least one
+  // partial; as many CTAs as there is room for (the plain kernels' partials alone: 304, two to an SM)
+  if (dtype == IGD_F64 && (path == 4 || (path == 0 && gram64_split_pays(n, a, b))) &&
+      (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
+    const int room = gram64_split_room(workspace_bytes, a, b);
+    if (room >= 1) {
+      g_gram_last = 4;
+      return gram64_split_launch(n, a, static_cast<const double*>(A), sa, b, static_cast<const double*>(B), sb, w, out,
+                                 accumulate, workspace, room, st);
+    }
   }
   // the pipelined kernel when rows are 16-byte aligned and outputs <= 64 x 64, else the register-tiled one
   const int e = path == 3 ? -1

@@ -309,11 +309,12 @@ __global__ void gram64_reduce_kernel(int nblocks, long long n, int a, const doub
 
 // At most 120 windows per warp (an int32 level sum takes 127 windows of at most 2^24): more than max_blocks CTAs
 // can take go in pieces, each with its own row exponents, added up in the output.  9.5 million points:
-// two pieces.
+// three pieces.
 int gram64_split_launch(long long n, int a, const double* A, long long sa, int b, const double* B, long long sb,
-                        const double* w, double* out, int accumulate, longlong2* part, int max_blocks, int* emax,
-                        cudaStream_t st) {
+                        const double* w, double* out, int accumulate, void* workspace, int max_blocks, cudaStream_t st) {
   constexpr long long MOST = 120, WINDOW = 32 * GW;
+  longlong2* const part = static_cast<longlong2*>(workspace);
+  int* const emax = reinterpret_cast<int*>(part + (long long)max_blocks * a * b);
   const int sms = device_sm_count();
   const int ty = (a + 15) / 16, tz = (b + 8 * GNT - 1) / (8 * GNT);
   const int sym = A == B && sa == sb && a == b;

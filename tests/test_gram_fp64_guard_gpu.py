@@ -67,3 +67,30 @@ def test_self_gram_with_an_overflowing_product():
     fine = np.isfinite(plain)
     assert fine[7].sum() == a - 1 and not fine[:, 7].any()  # (i, 7) multiplies the infinity, (7, j) does not
     assert np.all(np.abs(got - plain)[fine] <= 1e-12 * np.abs(plain)[fine] + 1e-9)
+
+
+@pytest.mark.parametrize("path", [0, 4])
+def test_workspace_alignment_and_size(path):
+    """A workspace aligned to a double, and one of the plain kernels' size, are taken as ever; one that is smaller is
+    refused."""
+
+    import torch
+
+    from isogriddft_gb300 import _lib
+
+    n, a, b = 1 << 18, 12, 9
+    g = torch.Generator("cuda").manual_seed(7)
+    A = torch.randn((a, n), dtype=torch.float64, device="cuda", generator=g)
+    B = torch.randn((b, n), dtype=torch.float64, device="cuda", generator=g)
+    w = torch.rand(n, dtype=torch.float64, device="cuda", generator=g)
+    want = ((A * w) @ B.T).cpu().numpy()
+    blocks = max(min(-(-n // 256), 608), min(-(-n // 16384), 4096))
+    plain = 8 * blocks * a * b  # one FP64 partial per block and output
+    full = int(_lib.call("igd_block_gram_workspace_bytes", n, a, b))
+    assert full <= 1.1 * plain
+    buf = torch.full((full // 8 + 4,), float("nan"), dtype=torch.float64, device="cuda")
+    for ws, size in ((buf[1:], full), (buf, plain), (buf[1:], plain), (buf, full)):
+        code, got, _ = _gram(A, B, w, path, ws, size)
+        assert code == 0 and np.all(np.abs(got - want) <= 1e-9)
+    assert bool(torch.isnan(buf[-3:]).all())
+    assert _gram(A, B, w, path, buf, plain - 8)[0] == _lib.IGD_ERR_ARG
