@@ -6,7 +6,8 @@
 // Rotation: out_j = sum_i A_i C1[i][j] + sum_i B_i C2[i][j]  (basis @ coeffs and
 // the two-part compressions of ks/eigensolver_jax.py:178-251).
 // FP32 data: products and per-thread sums (at most 64 points) in FP32, block
-// and cross-block accumulation in FP64; FP64 data: FP64 throughout.  Cross-block
+// and cross-block accumulation in FP64; FP64 data: FP64 throughout, or on large
+// grids exact products of digits with a bound on the error (blas64_split.cu).  Cross-block
 // sums are deterministic (per-block partials reduced in a second kernel).
 #include "blas64_split.cuh"
 #include "common.cuh"
@@ -22,10 +23,9 @@ thread_local int g_gram_path = 0;                   // igd_gram_select
 thread_local int g_gram_last = 0;                   // kernel of this thread's last Gram (1 tensor, 2 pipe, 3 tiled)
 // FP64: the splitting kernel takes about 22 clocks a point for every 16 x 24 outputs (splitting) plus
 // 8 (row exponents), the plain kernels 0.57 a point and output (FP64 pipe).  363609 points, plain /
-// split: 4 x 4 99 / 46 us (launch-bound plain grid), 8 x 8 99 / 48, 12 x 12 187 / 64, 21 x 21
-// 538 / 140, 34 x 34 1141 / 346; 2000003 points: 4 x 4 122 / 173, 8 x 8 376 / 202 (the plain kernel is
-// 8 % faster since its sums over lanes were shortened).  It would pay from
-// about a thousand points on (20001 points, 21 x 21: 72 / 29 us), but its correctly rounded sums
+// split: 4 x 4 111 / 57 us (launch-bound plain grid), 8 x 8 109 / 61, 12 x 12 176 / 82, 21 x 21
+// 505 / 161, 34 x 34 1068 / 374; 2000003 points: 4 x 4 122 / 198, 8 x 8 357 / 227, 21 x 21 2519 / 755.
+// It would pay from about a thousand points on, but its correctly rounded sums
 // differ from the plain ones in the last bit, and on small grids an eigensolve of a closure that is
 // not self-adjoint turns that into 1e-8 of an unconverged orbital; below the size where the FP32
 // Gram changes kernels too, the plain sums and with them the recorded iterates are kept.
@@ -58,12 +58,13 @@ __device__ __forceinline__ float narrow(double x, float) { return narrow(x); }
 // integer ALUs (35 x 35 over 870001 FP32 points 458 -> 367 us, 21 x 21 215 -> 179, over 20001 26 -> 22; FP64
 // 250 thousand points and fewer 7 to 12 %; unrolled by four or eight the large FP32 cases take a fifth more,
 // and tiles of 5 to 8 are slower throughout).
+// gram_tile_part: one such tile and slice, into part[slice].
 template <typename T, int TR>
-__global__ void __launch_bounds__(GTH) gram_tile_kernel(long long n, int a, int b, const T* __restrict__ A,
-                                                        long long sa, const T* __restrict__ B, long long sb,
-                                                        const double* __restrict__ w, double* __restrict__ part) {
+__device__ __forceinline__ void gram_tile_part(long long n, int a, int b, const T* __restrict__ A, long long sa,
+                                               const T* __restrict__ B, long long sb, const double* __restrict__ w,
+                                               double* __restrict__ part, int tile, int slice, int slices) {
   const int tb = (b + TR - 1) / TR;
-  const int i0 = (blockIdx.y / tb) * TR, j0 = (blockIdx.y % tb) * TR;
+  const int i0 = (tile / tb) * TR, j0 = (tile % tb) * TR;
   T acc[TR][TR];
 #pragma unroll
   for (int r = 0; r < TR; ++r)
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(GTH) gram_tile_kernel(long long n, int a, int 
     Br[r] = j0 + r < b ? B + (long long)(j0 + r) * sb : nullptr;
   }
 #pragma unroll 2
-  for (long long p = blockIdx.x * (long long)GTH + threadIdx.x; p < n; p += (long long)gridDim.x * GTH) {
+  for (long long p = slice * (long long)GTH + threadIdx.x; p < n; p += (long long)slices * GTH) {
     T av[TR], bv[TR];
     const T wp = w ? narrow(w[p], T()) : T(1);
 #pragma unroll
@@ -118,8 +119,57 @@ __global__ void __launch_bounds__(GTH) gram_tile_kernel(long long n, int a, int 
     static_assert(WARPS == 8, "the tree over eight warps");
     auto pair = [&](int q) { return scratch[q][e] + scratch[q + 4][e]; };
     if (r < a && c < b)
-      part[(long long)blockIdx.x * a * b + (long long)r * b + c] =
-          (pair(0) + pair(2)) + (pair(1) + pair(3));
+      part[(long long)slice * a * b + (long long)r * b + c] = (pair(0) + pair(2)) + (pair(1) + pair(3));
+  }
+}
+
+template <typename T, int TR>
+__global__ void __launch_bounds__(GTH) gram_tile_kernel(long long n, int a, int b, const T* __restrict__ A,
+                                                        long long sa, const T* __restrict__ B, long long sb,
+                                                        const double* __restrict__ w, double* __restrict__ part) {
+  gram_tile_part<T, TR>(n, a, b, A, sa, B, sb, w, part, blockIdx.y, blockIdx.x, gridDim.x);
+}
+
+// The listed tiles of a product that another kernel has formed, again: few tiles in as many slices as fill the
+// SMs, many in slices of the plain kernel's length.  The last block of a tile (its count goes up from 1) sums
+// the partials and writes the outputs marked in need (2: itself; 1: likewise, or from above the diagonal of a
+// symmetric product).
+template <int TR>
+__global__ void __launch_bounds__(GTH) gram_redo_kernel(long long n, int a, int b, const double* __restrict__ A,
+                                                        long long sa, const double* __restrict__ B, long long sb,
+                                                        const double* __restrict__ w, const Gram64Marks marks, int sym,
+                                                        double* part, long long partials, double* out, int accumulate) {
+  __shared__ int last;
+  const int count = *marks.listed, tb = (b + TR - 1) / TR;
+  if (count == 0) return;
+  const long long fill = gridDim.x / count, least = (n + GTH * GPT - 1) / (GTH * GPT);
+  const int slices = (int)min(max(min(fill, (n + 4 * GTH - 1) / (4 * GTH)), least), partials);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (long long item = blockIdx.x; item < (long long)count * slices; item += gridDim.x) {
+    const int tile = marks.list[item / slices];
+    gram_tile_part<double, TR>(n, a, b, A, sa, B, sb, w, part, tile, (int)(item % slices), slices);
+    if (threadIdx.x < 32) {
+      __threadfence();  // the partial, written by this warp, is visible before the count
+      __syncwarp();
+      if (threadIdx.x == 0) last = atomicAdd(marks.tiles + tile, 1) == slices;
+    }
+    __syncthreads();
+    if (last) {
+      __threadfence();
+      for (int e = warp; e < TR * TR; e += GTH / 32) {
+        const int r = (tile / tb) * TR + e / TR, c = (tile % tb) * TR + e % TR;
+        if (r >= a || c >= b) continue;
+        const long long at = (long long)r * b + c, mirror = (long long)c * b + r;
+        double sum = 0.0;
+        for (int k = lane; k < slices; k += 32) sum += __ldcg(part + (long long)k * a * b + at);
+        for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+        if (lane != 0) continue;
+        const int kind = marks.need[at];
+        if (kind == 2 || (kind == 1 && !(sym && r > c))) out[at] = accumulate ? out[at] + sum : sum;
+        if (sym && r < c && marks.need[mirror] == 1) out[mirror] = accumulate ? out[mirror] + sum : sum;
+      }
+    }
+    __syncthreads();  // `last` and the tile's scratch are used again
   }
 }
 
@@ -751,6 +801,14 @@ __global__ void jacobi_kernel(long long n, int k, const T* __restrict__ r, long 
 }
 
 }  // namespace
+
+int gram64_plain_redo(long long n, int a, const double* A, long long sa, int b, const double* B, long long sb,
+                      const double* w, double* out, int accumulate, int sym, const Gram64Marks& marks, double* part,
+                      long long partials, cudaStream_t st) {
+  gram_redo_kernel<GRAM64_TILE><<<2 * device_sm_count(), GTH, 0, st>>>(n, a, b, A, sa, B, sb, w, marks, sym, part,
+                                                                       partials, out, accumulate);
+  return launch_status();
+}
 }  // namespace igd
 
 using namespace igd;

@@ -94,3 +94,55 @@ def test_workspace_alignment_and_size(path):
         assert code == 0 and np.all(np.abs(got - want) <= 1e-9)
     assert bool(torch.isnan(buf[-3:]).all())
     assert _gram(A, B, w, path, buf, plain - 8)[0] == _lib.IGD_ERR_ARG
+
+
+def _wide(kind, n):
+    """Rows A (5, n) and B (4, n), whose products are far below max|a| max|b| at every point."""
+
+    import torch
+
+    r = torch.linspace(0.0, 60.0, n, dtype=torch.float64, device="cuda")
+    g = torch.Generator("cuda").manual_seed(2)
+    A = torch.randn((5, n), dtype=torch.float64, device="cuda", generator=g)
+    B = torch.randn((4, n), dtype=torch.float64, device="cuda", generator=g)
+    if kind == "opposite":  # localised at opposite ends
+        A *= torch.exp(-r)
+        B *= torch.exp(r - 60.0)
+    elif kind == "spike":  # one value of A far above the rest, where B is zero
+        A[:, 5] = 1e8
+        B[:, 5] = 0.0
+    elif kind == "weight":  # one weight far above the rest, where A is zero
+        A[:, 9] = 0.0
+        B[:, 9] = 1e9
+    elif kind == "disjoint":
+        A[:, n // 2:] = 0.0
+        B[:, :n // 2] = 0.0
+    elif kind == "zero":
+        A[1] = 0.0
+        B[2] = 0.0
+    return A, B
+
+
+# one window, several, and the size from which the automatic choice is the splitting kernel
+@pytest.mark.parametrize("n", [50, 5003, 1 << 18])
+@pytest.mark.parametrize("kind", ["normal", "opposite", "spike", "weight", "disjoint", "zero"])
+def test_split_gram_keeps_the_plain_accuracy(n, kind):
+    """Every output to the plain kernels' bound, relative to sum |a w b|: 2^-53 for each of at most 64 products of a
+    thread, their sums, the tree over 256 threads and the sum over at most 608 blocks (10 steps): 2^-45 in all."""
+
+    import torch
+
+    A, B = _wide(kind, n)
+    w = torch.rand(n, dtype=torch.float64, device="cuda") + 1e-3
+    for X, Y, ww in ((A, B, w), (A, B, None), (A, A, w)):
+        for path in (4, 0):
+            code, got, last = _gram(X, Y, ww, path)
+            assert code == 0 and (path == 0 or last == 4)
+            x, y = X.cpu().numpy().astype(np.longdouble), Y.cpu().numpy().astype(np.longdouble)
+            y = y * (ww.cpu().numpy() if ww is not None else 1)
+            want, scale = x @ y.T, np.abs(x) @ np.abs(y).T
+            assert np.all(np.abs(got - want) <= 2.0**-45 * scale), (
+                last, float(np.max(np.abs(got - want) / (scale + (scale == 0)))))
+            # added to a non-zero result, outputs of every route once
+            _, twice, _ = _gram(X, Y, ww, path, out=torch.full(got.shape, 0.5, dtype=torch.float64, device="cuda"))
+            assert np.array_equal(twice, 0.5 + got)
