@@ -136,10 +136,10 @@ int igd_hpsi_legacy(int dtype, int nx, int ny, int nz, const double* axis_coeffs
  * max |f - A u| (interior).  Returns IGD_ERR_BREAKDOWN on Krylov breakdown;
  * reaching max_iterations is reported through info, not as an error. */
 long long igd_poisson_workspace_bytes(int precision, long long n);
-/* Test hook for the calling host thread: 0 = the inner FP32 solve of the mixed
- * Poisson path uses the fused iteration (dot products from the stencil
- * epilogue, scalars recomputed in the vector kernels) wherever the whole-row
- * operator applies, 1 = the unfused iteration.  No reference counterpart. */
+/* Test hook for the calling host thread: 0 = solves on monitor grids use the
+ * fused iteration (dot products from the stencil epilogue, scalars recomputed
+ * in the vector kernels) wherever an operator with that epilogue applies, 1 =
+ * the unfused iteration.  No reference counterpart. */
 int igd_poisson_select(int path);
 /* The JAX route of the monitor-grid solve (poisson/poisson_jax.py:675-750):
  * preconditioned CG on the interior -L (production closure, FP64) from x = 0,

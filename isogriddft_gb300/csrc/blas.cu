@@ -355,8 +355,12 @@ constexpr int RTH = 256;
 // one and 7.4 with two over 117649 points; over 40000, 5.3 with one.
 constexpr long long ROT_PAIR_POINTS = 100000;
 // The pipeline's batches and its lower line: 22 rows to 20 columns over 363608 points take 15.2 us there and
-// 14.9 in the register kernel, 50 to 35 over 10^6 124 and 160, 19 to 12 23 and 37 (rotate_kernel).  Its
-// coefficients, rows x columns, have to leave room for two CTAs on an SM.
+// 14.9 in the register kernel, 50 to 35 over 10^6 124 and 160, 19 to 12 23 and 37 (rotate_kernel).  Up to
+// ROT_PIPE_COEF coefficients, rows x columns, fit beside the ring.  Up to 16 columns the ring is 96 KB, and from
+// about 16 KB of coefficients on (at the padded width) a CTA is alone on its SM: slower, but still ahead of
+// rotate_kernel.  2^19 points, pipeline / rotate_kernel: 341 rows to 12 columns 177 / 300 us (two CTAs), 512 to
+// 12 300 / 439 (one), 256 to 13 162 / 230 (two), 470 to 13 328 / 407 (one), 384 to 16 275 / 335 (one), 1536 to 4
+// 616 / 839 (one), 6144 to 1 2407 / 10155 (one).
 constexpr int ROT_STAGES = 3, ROT_ROWS = 8;
 constexpr long long ROT_PIPE_POINTS = 1 << 19, ROT_PIPE_COEF = 6 * 1024;
 

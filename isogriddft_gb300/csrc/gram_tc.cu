@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const long long G = gridDim.x;
   const long long J = g.stages > blockIdx.x ? (g.stages - blockIdx.x + G - 1) / G : 0;  // stages of this CTA
 
-  // raw tile of ring slot q: A chunks, B chunks, w; split buffer: A hi, A lo, B hi, B lo
+  // raw tile of ring slot q: A chunks, B chunks; split buffer: A hi, A lo, B hi, B lo
   auto slotA = [&](int q) { return base + (size_t)LS * g.split_bytes + (size_t)q * g.slot_bytes; };
   auto slotB = [&](int q) { return slotA(q) + (size_t)g.s * g.a_rows * 128; };
   auto splitA = [&](int u) { return base + (size_t)u * g.split_bytes; };
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       return v;
     };
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    // epilogue of window `win`: TMEM diagonal blocks -> FP64 registers
+    // epilogue of window `win`: TMEM diagonal blocks -> compensated FP32 sums in registers
     auto flush = [&](long long win) -> bool {
       const int buf = (int)(win & 1);
       // lanes agree before the warp-collective TMEM loads (an abort may reach them unevenly)
