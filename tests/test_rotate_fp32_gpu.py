@@ -76,3 +76,22 @@ def test_coefficients_beyond_shared_memory_are_refused(c, most):
         else:
             with pytest.raises(Exception):
                 _rotate(*args, 0)
+
+
+@pytest.mark.parametrize("a,b,c", [(512, 0, 12), (300, 170, 13), (1536, 0, 4)])
+def test_many_rows_to_few_columns(a, b, c):
+    """Coefficients that leave one CTA of the pipeline on an SM."""
+    n = EDGE + 4
+    g = torch.Generator(device="cuda").manual_seed(a + b + c)
+    rnd = lambda *s, **k: torch.randn(*s, generator=g, device="cuda", **k)
+    A, C1, C2 = rnd(a, n), rnd(a, c, dtype=torch.float64), rnd(max(b, 1), c, dtype=torch.float64)
+    B = rnd(b, n) if b else None
+    out = rnd(c, n)
+    _rotate(A, C1, B, C2, out, 0)
+    bound = torch.zeros(c, n, device="cuda", dtype=torch.float64)
+    want = torch.zeros_like(bound)
+    for X, C in ((A, C1), (B, C2)):
+        for r in range(0, X.shape[0] if X is not None else 0, 64):
+            want += C[r:r + 64].T @ X[r:r + 64].double()
+            bound += C[r:r + 64].T.abs() @ X[r:r + 64].double().abs()
+    assert bool(((out.double() - want).abs() <= (a + b + 3) * 2.0**-24 * bound).all())
