@@ -10,10 +10,11 @@
 // products of two digits are integers of at most 2^16; an FP32 accumulator takes 256 of them
 // without rounding, so the sums of all digit pairs of one weight (28 pairs in seven levels; lower
 // ones are below 2^-58 of the largest product) are exact integers over a window of 32 points,
-// collected as int32 and turned into FP64 once per output.  Splitting is integer work on the otherwise
-// idle ALUs (about 35 instructions a value) and bounds the kernel; the products go through mma.sync
-// m16n8k16 (FP16 in, FP32 out), whose fragments are the splitting's own registers (the tensor pipe is
-// mostly idle: operands staged for tcgen05 would only add traffic).
+// collected as int32 and turned into FP64 once per output.  Splitting is integer work (about 35
+// instructions a value) and bounds the kernel: integer pipe 48 % and issue 47 % active with two CTAs of
+// four warps on an SM.  The products go through mma.sync m16n8k16 (FP16 in, FP32 out), whose fragments are
+// the splitting's own registers (the tensor pipe is 30 % active: operands staged for tcgen05 would only add
+// traffic).
 //
 // What is lost are bits below 2^-61 of the row's largest value: nothing of the values within 2^-9 of
 // it, everything of those below 2^-61.  Against the sum of |a w b|, on which the plain kernels' rounding

@@ -46,6 +46,12 @@ def test_split_gram_above_nine_million_points():
     assert last == 4 and np.all(np.abs(got - plain) <= 2.0**-44 * scale.cpu().numpy())
     _, more, _ = _gram(A, B, w, 4, out=torch.full((3, 2), 1.0, dtype=torch.float64, device="cuda"))
     assert np.all(np.abs(more - 1.0 - got) <= 2.0**-50 * np.abs(got) + 2.0**-50)
+    # rows that do not overlap: zero in every piece, by either route
+    A[0, n // 2:] = 0.0
+    B[0, :n // 2] = 0.0
+    (_, got, _), (_, plain, _) = _gram(A, B, w, 4), _gram(A, B, w, 3)
+    scale = (A.abs() * w) @ B.abs().T
+    assert got[0, 0] == 0.0 and np.all(np.abs(got - plain) <= 2.0**-44 * scale.cpu().numpy())
 
 
 def test_self_gram_with_an_overflowing_product():
